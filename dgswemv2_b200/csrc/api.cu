@@ -75,10 +75,7 @@ int make_l2_rule(L2Rule& R, std::string& err) {
     return DGSW_OK;
 }
 
-__global__ void advance_clock_kernel(DevClock* c, double dt) {
-    c->t += dt;  // ESSPRKStepper::operator++ (explicit_ssp_rk_stepper.hpp:55-58)
-    c->step += 1;
-}
+__global__ void step_time_kernel(const __grid_constant__ TimeArgs T) { form_step_time(&T, (int)blockIdx.x); }
 
 }  // namespace
 
@@ -137,7 +134,8 @@ struct dgsw_rkdg_s {
     DBuf<unsigned char> wet[2];
     int wet_cur = 0;
     DBuf<DevStatus> status;
-    DBuf<DevClock> clock;
+    DBuf<DevClock> clock;  // two copies, keyed by qswap (StageArgs::time)
+    DBuf<double> fval;     // tide / flow values of both copies
     DBuf<double> red;  // reduction partials
     DBuf<unsigned char> limited;
     DBuf<int> nbr;     // neighbours per face, device order (limiter)
@@ -204,6 +202,56 @@ namespace {
 // steps per multi-step graph
 constexpr int GRAPH_MULTI = 8;
 
+size_t forcing_values(const dgsw_rkdg_s* h) {  // per forcing value set
+    return h->fface.n * (size_t)h->tb.ng;
+}
+
+// the forcing value set of stage s: stages with one time offset share a set
+int forcing_set(const dgsw_rkdg_s* h, int s, TimeArgs* T = nullptr) {
+    int n = 0, mine = 0;
+    for (int k = 0; k < h->ns; ++k) {
+        int first = 0;
+        while (h->rk.drk[first] != h->rk.drk[k]) ++first;
+        if (first != k) continue;
+        if (T) T->set_stage[n] = k;
+        if (h->rk.drk[k] == h->rk.drk[s]) mine = n;
+        ++n;
+    }
+    if (T) T->nsets = n;
+    return mine;
+}
+
+// arguments that form copy `copy` of the step's time data
+TimeArgs time_args(dgsw_rkdg_s* h, int copy) {
+    TimeArgs T;
+    std::memset(&T, 0, sizeof(T));
+    T.dt = h->cfg.dt;
+    for (int s = 0; s < h->ns; ++s) T.off[s] = h->cfg.dt * h->rk.drk[s];
+    T.nstages = h->ns;
+    T.fn_set = h->cfg.function_set;
+    for (int i = 0; i < 16; ++i) T.fn_params[i] = h->cfg.fn_params[i];
+    // ESSPRKStepper keeps ramp = 1 when Utilities::almost_equal(ramp_duration, 0)
+    T.ramp_on = std::fabs(h->cfg.ramp_duration) < std::numeric_limits<double>::epsilon() * 100 ? 0 : 1;
+    T.ramp_duration = h->cfg.ramp_duration;
+    T.fface = h->fface.p;
+    T.fcon = h->fcon.p;
+    T.n_forced = (int)h->fface.n;
+    T.ng = h->tb.ng;
+    forcing_set(h, 0, &T);
+    T.next = h->clock.p + copy;
+    T.fval = h->fval.p + (size_t)copy * T.nsets * forcing_values(h);
+    return T;
+}
+
+// the current step's time data from the host's t and step
+cudaError_t write_step_time(dgsw_rkdg_s* h) {
+    TimeArgs T = time_args(h, h->qswap);
+    T.t0 = h->t;
+    T.step0 = h->step;
+    step_time_kernel<<<step_time_blocks(T, 128), 128, 0, h->stream>>>(T);
+    return cudaGetLastError();
+}
+
 template <typename Real>
 void fill_stage_args(dgsw_rkdg_s* h, int s, StageArgs<Real>& A) {
     std::memset(&A, 0, sizeof(A));
@@ -260,8 +308,13 @@ void fill_stage_args(dgsw_rkdg_s* h, int s, StageArgs<Real>& A) {
     A.ref_of_dev = h->ref_of_dev.p;
     A.baryctr = h->cfg.slope_limiting ? h->baryctr.p : nullptr;
     A.status = h->status.p;
-    A.clock = h->clock.p;
-    A.drk_s = h->cfg.dt * h->rk.drk[s];
+    A.clock = h->clock.p + h->qswap;
+    if (s + 1 == h->ns) {
+        A.time = time_args(h, 1 - h->qswap);
+        A.time.cur = A.clock;
+        A.n_time = step_time_blocks(A.time, h->tile);
+    }
+    A.ntiles = (int)h->tiling.ntiles;
     A.stage_index = s;
     A.nstages = h->ns;
     A.ne = (int)h->ne;
@@ -277,11 +330,11 @@ void fill_stage_args(dgsw_rkdg_s* h, int s, StageArgs<Real>& A) {
     A.friction = h->cfg.bottom_friction;
     A.friction_cf = h->cfg.friction_cf;
     A.manning = (const Real*)h->manning;
-    A.fface = h->fface.p;
-    A.fcon = h->fcon.p;
-    // ESSPRKStepper keeps ramp = 1 when Utilities::almost_equal(ramp_duration, 0)
-    A.ramp_on = std::fabs(h->cfg.ramp_duration) < std::numeric_limits<double>::epsilon() * 100 ? 0 : 1;
-    A.ramp_duration = h->cfg.ramp_duration;
+    {
+        TimeArgs T;
+        const int set = forcing_set(h, s, &T);
+        A.fval = h->fval.p + ((size_t)h->qswap * T.nsets + set) * forcing_values(h);
+    }
     A.went_dry = h->went_dry.p;
     // tile order alternates from stage to stage, across steps too (qswap flips once per step and keys
     // the step graphs), so that each stage starts where the previous one ended
@@ -428,7 +481,7 @@ __global__ void record_labels_kernel(const unsigned char* limited, const int* re
 
 cudaError_t split_form(dgsw_rkdg_s* h, int s);
 
-// one RK stage: stage kernel, (clock on the last stage), indicator, limiter, wet flag buffer flip
+// one RK stage: stage kernel (with the clock on the last stage), indicator, limiter, wet flag buffer flip
 cudaError_t enqueue_stage(dgsw_rkdg_s* h, int s, int64_t& launches, const StageRecord* rec = nullptr) {
     const bool timed = h->kt_on && h->kt_used + 2 <= h->kt_ev.size();
     if (timed) {
@@ -446,10 +499,6 @@ cudaError_t enqueue_stage(dgsw_rkdg_s* h, int s, int64_t& launches, const StageR
     h->wet_cur = 1 - h->wet_cur;
     int s_out = s + 1;
     if (s + 1 == h->ns) {
-        advance_clock_kernel<<<1, 1, 0, h->stream>>>(h->clock.p, h->cfg.dt);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        ++launches;
         std::swap(h->Q[0], h->Q[h->ns]);  // UpdateState's swap of q_0 and q_ns
         h->qswap ^= 1;
         s_out = 0;
@@ -1000,8 +1049,16 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
         std::memset(&z, 0, sizeof(z));
         z.nan_key = ~0ull;
         cudaMemcpy(h->status.p, &z, sizeof(z), cudaMemcpyHostToDevice);
-        if ((e = h->clock.alloc(1)) != cudaSuccess) return cleanup_fail("alloc", e);
-        cudaMemset(h->clock.p, 0, sizeof(DevClock));
+        if ((e = h->clock.alloc(2)) != cudaSuccess) return cleanup_fail("alloc", e);
+        {
+            TimeArgs T;
+            forcing_set(h, 0, &T);
+            if ((e = h->fval.alloc(2 * (size_t)T.nsets * forcing_values(h))) != cudaSuccess) return cleanup_fail("alloc", e);
+            h->device_bytes += (int64_t)h->fval.n * 8;
+        }
+        // the forcing data's copies above ran on the default stream, which the handle's stream does not wait for
+        if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess || (e = write_step_time(h)) != cudaSuccess)
+            return cleanup_fail("clock", e);
         if ((e = h->red.alloc(reduction_partials(h->ne))) != cudaSuccess) return cleanup_fail("alloc", e);
         {
             static L2Rule Rh;
@@ -1461,6 +1518,7 @@ int32_t dgsw_rkdg_destroy(dgsw_handle h) {
     h->wet[1].release();
     h->status.release();
     h->clock.release();
+    h->fval.release();
     h->red.release();
     h->l2rule.release();
     h->staging.release();
@@ -1523,8 +1581,7 @@ int32_t dgsw_rkdg_init_state(dgsw_handle h) {
     h->t = 0.0;
     h->step = 0;
     h->stage = 0;
-    DevClock c = {0.0, 0};
-    CUDA_TRY(cudaMemcpyAsync(h->clock.p, &c, sizeof(c), cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(write_step_time(h));
     int rc = upload_state(h, q.data());
     if (rc) return rc;
     return upload_wet(h, wet.data());

@@ -71,10 +71,90 @@ struct DevStatus {
     unsigned int pad;
 };
 
+// What a stage needs of its time (t + dt drk[s]): the function set's time factors and the forcing ramp
+struct StageTime {
+    dgsw_fn_time ft;
+    double ramp;
+};
+
 struct DevClock {
     double t;  // time at the start of the current step (ESSPRKStepper::t)
     long long step;
+    StageTime at[DGSW_RK_MAX_STAGES];  // per stage of the current step
 };
+
+constexpr int FORCE_STRIDE_DEV = 9;
+
+// Everything that depends on time alone, formed once per step for the next one: the clock itself, each
+// stage's time factors (FP64 sines and cosines) and the tide / flow values at the forced faces' Gauss points.
+// There are two copies, keyed by the step's parity: a step reads one while extra CTAs of its last stage's
+// launch write the other, so neither a launch of its own nor the stage's CTAs wait for that arithmetic.
+// Stages with the same offset drk share one set of forcing values (all of them in the reference's tables).
+struct TimeArgs {
+    double dt;
+    double off[DGSW_RK_MAX_STAGES];  // dt drk[s]
+    int nstages;
+    int fn_set;
+    double fn_params[16];
+    int ramp_on;           // ramp_duration not almost zero
+    double ramp_duration;  // days
+    // tide / flow boundary forcing: per forced face its first constituent entry and count; per entry
+    // frequency, forcing factor, equilibrium argument, amplitude[3] and phase[3] at the Gauss points
+    const int2* fface;
+    const double* fcon;
+    int n_forced, ng;
+    int nsets;                          // forcing value sets
+    int set_stage[DGSW_RK_MAX_STAGES];  // the first stage of each set
+    const DevClock* cur;                // advance from this copy (null: write `t0`, `step0` as they are)
+    double t0;
+    long long step0;
+    DevClock* next;
+    double* fval;  // [nsets][n_forced][ng] written for `next`
+};
+
+// the ramp of ESSPRKStepper::operator++, explicit_ssp_rk_stepper.hpp:49-65 (1 without a ramp)
+__device__ __forceinline__ double forcing_ramp(const TimeArgs& T, double t) {
+    return T.ramp_on ? tanh(2.0 * (t / 86400.0) / T.ramp_duration) : 1.0;
+}
+
+// block 0: the clock and the stages' time factors; the others: one forcing value per thread,
+// sum_con ramp * forcing_fact * amplitude_gp * cos(frequency * t + (equilib_arg - phase_gp) * PI / 180)
+// with the reference's PI = 3.14159265359 (rkdg_swe_bc_tide.hpp:73-100, rkdg_swe_bc_flow.hpp:72-102), in FP64
+// in both precisions. Out of line: only the extra CTAs of a step's last stage come here.
+static __device__ __noinline__ void form_step_time(const TimeArgs* Tp, int block) {
+    const TimeArgs& T = *Tp;
+    const double t = T.cur ? T.cur->t + T.dt : T.t0;  // ESSPRKStepper::operator++ (:55-58)
+    if (block == 0) {
+        const int s = threadIdx.x;
+        if (s < T.nstages) {
+            T.next->at[s].ft = dgsw_fn_prepare(T.fn_set, T.fn_params, t + T.off[s]);
+            T.next->at[s].ramp = forcing_ramp(T, t + T.off[s]);
+        }
+        if (s == 0) {
+            T.next->t = t;
+            T.next->step = T.cur ? T.cur->step + 1 : T.step0;
+        }
+        return;
+    }
+    const int per_set = T.n_forced * T.ng;
+    const int i = (block - 1) * (int)blockDim.x + (int)threadIdx.x;
+    if (i >= T.nsets * per_set) return;
+    constexpr double REF_PI = 3.14159265359;
+    const int set = i / per_set, gp = i % T.ng;
+    const double ts = t + T.off[T.set_stage[set]];
+    const double ramp = forcing_ramp(T, ts);
+    const int2 fc = T.fface[(i % per_set) / T.ng];
+    double acc = 0.0;
+    for (int c = 0; c < fc.y; ++c) {
+        const double* r = T.fcon + (size_t)(fc.x + c) * FORCE_STRIDE_DEV;
+        acc += ramp * r[1] * r[3 + gp] * cos(r[0] * ts + (r[2] - r[6 + gp]) * REF_PI / 180.0);
+    }
+    T.fval[i] = acc;
+}
+// CTAs of `threads` threads that form_step_time takes
+inline int step_time_blocks(const TimeArgs& T, int threads) {
+    return 1 + (T.nsets * T.n_forced * T.ng + threads - 1) / threads;
+}
 
 // Real is the arithmetic type of the stage (FP32 bulk or FP64); the stage states and stored stage
 // solutions are FP64 in both, so that the RK update does not accumulate FP32 rounding from stage to stage
@@ -104,8 +184,10 @@ struct StageArgs {
     const int* ref_of_dev;
     double* baryctr;  // [3][ne_pad] barycentre values of the new state for the slope limiter, or null
     DevStatus* status;
-    const DevClock* clock;
-    double drk_s;  // stage-time offset of this stage (t + dt*drk[s])
+    const DevClock* clock;  // this step's copy
+    TimeArgs time;          // the next step's copy, formed by `n_time` extra CTAs of the last stage's launch
+    int n_time;
+    int ntiles;
     int stage_index, nstages;  // this stage and the stages per step (the NaN report's stage counter)
     int ne;
     int ne_pad;
@@ -120,12 +202,7 @@ struct StageArgs {
     int friction;
     double friction_cf;
     const Real* manning;  // [ne_pad] g n^2 per element (Manning)
-    // tide / flow boundary forcing: per forced face its first constituent entry and count; per entry
-    // frequency, forcing factor, equilibrium argument, amplitude[3] and phase[3] at the Gauss points
-    const int2* fface;
-    const double* fcon;
-    int ramp_on;           // ramp_duration not almost zero
-    double ramp_duration;  // days
+    const double* fval;   // [n_forced][NG] this stage's tide / flow values at the forced faces' Gauss points
     // levee interface fluxes of this stage, [n_levee][2][3][NG] (levee.cu): in side, then ex side
     const double* levF;
     unsigned char* went_dry;  // [ne] wet_dry_state.went_completely_dry of the last wet/dry pass, or null
@@ -147,8 +224,6 @@ struct StageArgs {
     Real* q0lo_out;                         // new carried state, trailing part (last stage)
     int last;                               // this is the step's last stage
 };
-
-constexpr int FORCE_STRIDE_DEV = 9;
 
 // ------------------------------------------------------------------------------------------------
 // LLF flux, rkdg_swe_LLF_flux.hpp:7-60 (sp applied to the in-side normal flux only, as there)
@@ -273,35 +348,26 @@ __device__ __noinline__ Val3<Real> fn_eval_dev(int id, const double* P, const dg
     return Val3<Real>{out[0], out[1], out[2]};
 }
 
-// Ghost states of the boundaries with data, out of line (one call site per Gauss point):
+// Ghost states of the boundaries with data, out of line (one call site per Gauss point; inlined, the p = 1
+// FP32 kernels spill 50-70 bytes per thread and the wet/dry bowl step took 10 % longer):
 // BC::Function (kind 2): ic_q(t, x_gp) (rkdg_swe_bc_function.hpp:33-50);
-// BC::Tide (kind 3) and BC::Flow (kind 4) (rkdg_swe_bc_tide.hpp:73-100, rkdg_swe_bc_flow.hpp:72-102), in
-// FP64 in both precisions: the forced value is
-// sum_con ramp * forcing_fact * amplitude_gp * cos(frequency * t + (equilib_arg - phase_gp) * PI / 180)
-// with the reference's PI = 3.14159265359 and ramp = tanh(2 (t / 86400) / ramp_duration)
-// (ESSPRKStepper::operator++, explicit_ssp_rk_stepper.hpp:49-65; 1 without a ramp). A tide sets the
-// ghost surface elevation to it and keeps the interior momentum; a flow keeps the interior elevation
-// and sets the ghost momentum to it times the outward normal. fi is the face's forcing record.
+// BC::Tide (kind 3) and BC::Flow (kind 4) (rkdg_swe_bc_tide.hpp:73-100, rkdg_swe_bc_flow.hpp:72-102) from the
+// stage's forcing value (form_step_time): a tide sets the ghost surface elevation to it and keeps the
+// interior momentum; a flow keeps the interior elevation and sets the ghost momentum to it times the
+// outward normal. fi is the face's forcing record.
 template <typename Real>
-__device__ __noinline__ Val3<Real> boundary_ghost(const StageArgs<Real>* Ap, const dgsw_fn_time* T, int kind,
-                                                  int fi, int gp, double t, Real x, Real y, Real qi0, Real qi1,
-                                                  Real qi2, Real nx, Real ny) {
+__device__ __noinline__ Val3<Real> boundary_ghost(const StageArgs<Real>* Ap, const dgsw_fn_time* T, int kind, int fi,
+                                                  int gp, int ng, Real x, Real y, Real qi0, Real qi1, Real qi2,
+                                                  Real nx, Real ny) {
     const StageArgs<Real>& A = *Ap;
     if (kind == 2) {
         Real qe[3];
         dgsw_fn_eval<Real>(A.fn_set, A.fn_params, *T, 0, x, y, qe);
         return Val3<Real>{qe[0], qe[1], qe[2]};
     }
-    constexpr double REF_PI = 3.14159265359;
-    const double ramp = A.ramp_on ? tanh(2.0 * (t / 86400.0) / A.ramp_duration) : 1.0;
-    const int2 fc = A.fface[fi];
-    double acc = 0.0;
-    for (int c = 0; c < fc.y; ++c) {
-        const double* r = A.fcon + (size_t)(fc.x + c) * FORCE_STRIDE_DEV;
-        acc += ramp * r[1] * r[3 + gp] * cos(r[0] * t + (r[2] - r[6 + gp]) * REF_PI / 180.0);
-    }
-    if (kind == 4) return Val3<Real>{qi0, (Real)acc * nx, (Real)acc * ny};
-    return Val3<Real>{(Real)acc, qi1, qi2};
+    const Real f = (Real)A.fval[fi * ng + gp];
+    if (kind == 4) return Val3<Real>{qi0, f * nx, f * ny};
+    return Val3<Real>{f, qi1, qi2};
 }
 
 // the Manning friction factor g n^2 / h^(1/3), bounded below by the Chezy coefficient (swe_source.hpp:37-42);
@@ -761,19 +827,21 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
 
     // odd stages walk the tiles backwards: they start on the tiles the previous stage wrote last,
     // whose states are still in L2 (tiles are independent, so the results do not change)
-    const int tile = A.reverse ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+    if ((int)blockIdx.x >= A.ntiles) {
+        form_step_time(&A.time, (int)blockIdx.x - A.ntiles);
+        return;
+    }
+    const int tile = A.reverse ? A.ntiles - 1 - (int)blockIdx.x : (int)blockIdx.x;
     const int e0 = tile * TILE;
     const int nloc = min(TILE, A.ne - e0);
     const int tid = threadIdx.x;
     const int d = e0 + tid;
     const bool active = tid < nloc;
     const int P_ = A.ne_pad;
-    const double t_stage = A.clock->t + A.drk_s;  // ESSPRKStepper::GetTimeAtCurrentStage
     const Real g = (Real)A.g;
     const double* __restrict__ qs = A.qk[A.nterms - 1];  // this stage's state
-    // the stage's time factors, once per CTA in shared memory (the out-of-line helpers read them there)
-    __shared__ dgsw_fn_time sFT;
-    if (threadIdx.x == 0) sFT = dgsw_fn_prepare(A.fn_set, A.fn_params, t_stage);
+    // the stage's time factors (ESSPRKStepper::GetTimeAtCurrentStage), formed during the previous step
+    const dgsw_fn_time& FT = A.clock->at[A.stage_index].ft;
     // the face traces' basis values at the edge Gauss points, [face][mode][gp], for phase 3's lift and the
     // halo traces: the elements of a warp visit their faces in different orders, and compile-time tables per
     // face split the warp into one branch per face. Measured per step (bit-identical results): FP32 at p = 2
@@ -794,8 +862,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
         });
         sfphi[threadIdx.x] = c;
     }
-    __syncthreads();
-    const dgsw_fn_time& FT = sFT;
+    if (rt_face) __syncthreads();
     // the manufactured sine set's source inline, in both precisions; other sets go through fn_eval_dev
     const bool sine_set = FSRC && A.fn_set == DGSW_FN_MANUFACTURED_SINE;
     SineSrc<Real> SS;
@@ -1359,7 +1426,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
                     // function, tide and flow boundaries (a tide / flow face's b slot holds -2 - its
                     // forcing record)
                     const Val3<Real> r =
-                        boundary_ghost<Real>(&A, &FT, kind, -2 - sb, gp, t_stage, (Real)(xa * wa_ + xb * wb_),
+                        boundary_ghost<Real>(&A, &FT, kind, -2 - sb, gp, NG, (Real)(xa * wa_ + xb * wb_),
                                              (Real)(ya * wa_ + yb * wb_), qi[0], qi[1], qi[2], nx, ny);
                     qe[0] = r.v0, qe[1] = r.v1, qe[2] = r.v2;
                 }
@@ -1681,7 +1748,7 @@ cudaError_t launch_stage_impl(const StageArgs<Real>& A, int ntiles, int max_halo
                                : Smem<P, Real, WD>::off_halo(TILE, max_halo, max_edges);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)ntiles, TILE, smem, s>>>(A, max_halo, max_edges);
+    kern<<<(unsigned)(ntiles + A.n_time), TILE, smem, s>>>(A, max_halo, max_edges);
     return cudaGetLastError();
 }
 
