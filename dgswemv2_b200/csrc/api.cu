@@ -111,8 +111,9 @@ struct dgsw_rkdg_s {
     std::vector<void*> D;     // [ns], D[0] unused
     std::vector<void*> DSOL;  // FP32 stored stage solutions (only where needed)
     void* bath = nullptr;  // [3][ne_pad] bathymetry modes of the linear part
-    void* geo = nullptr;   // [5][ne_pad] J^-1 and |J|
-    void* egeo = nullptr;  // [3][n_edges] edge normal and half length
+    void* geo = nullptr;    // [4][ne_pad] J^-1
+    DBuf<int> fmeta;        // [3][ne_pad] face kinds and slots
+    void* fw = nullptr;     // [3][ne_pad] half face length over |J|
     void* manning = nullptr;  // [ne_pad] g n^2 per element (Manning friction only)
     Forcing forcing;
     DBuf<int2> fface;      // tide / flow forcing records
@@ -125,10 +126,8 @@ struct dgsw_rkdg_s {
     DBuf<double> post;             // output values for the writers (allocated on first use)
     DBuf<unsigned char> post_flags;
     DBuf<int2> halo;
-    DBuf<int> tile_halo_off;
-    DBuf<int> enodes, tile_edge_off, ref_of_dev;
-    DBuf<int2> eslot;
-    DBuf<int4> edges;
+    DBuf<int4> tiles;
+    DBuf<int> enodes, ref_of_dev;
     DBuf<double2> xy;
     DBuf<double> nz;
     DBuf<unsigned char> wet[2];
@@ -296,13 +295,10 @@ void fill_stage_args(dgsw_rkdg_s* h, int s, StageArgs<Real>& A) {
     A.bath = (const Real*)h->bath;
     A.geo = (const Real*)h->geo;
     A.enodes = h->enodes.p;
-    A.eslot = h->eslot.p;
-    A.edges = h->edges.p;
-    A.egeo = (const Real*)h->egeo;
-    A.tile_edge_off = h->tile_edge_off.p;
+    A.fmeta = h->fmeta.p;
+    A.fw = (const Real*)h->fw;
+    A.tiles = h->tiles.p;
     A.halo = h->halo.p;
-    A.tile_halo_off = h->tile_halo_off.p;
-    A.n_edges = (int)(h->tiling.edges.size() / 4);
     A.xy = h->xy.p;
     A.nz = h->nz.p;
     A.ref_of_dev = h->ref_of_dev.p;
@@ -342,27 +338,27 @@ void fill_stage_args(dgsw_rkdg_s* h, int s, StageArgs<Real>& A) {
 }
 
 cudaError_t launch_stage_any(dgsw_rkdg_s* h, const StageArgs<double>& A, int mode) {
-    const int nt = (int)h->tiling.ntiles, mh = h->tiling.max_halo, me = h->tiling.max_edges;
+    const int nt = (int)h->tiling.ntiles, mh = h->tiling.max_halo;
     if (h->uncapped) mode |= STAGE_MODE_UNCAPPED;
     if (h->occ)
-        return h->cfg.p == 1 ? launch_stage_p1_f64_occ(A, h->tile, nt, mh, me, mode, h->stream)
-                             : launch_stage_p2_f64_occ(A, h->tile, nt, mh, me, mode, h->stream);
-    return h->cfg.p == 1 ? launch_stage_p1_f64(A, h->tile, nt, mh, me, mode, h->stream)
-                         : launch_stage_p2_f64(A, h->tile, nt, mh, me, mode, h->stream);
+        return h->cfg.p == 1 ? launch_stage_p1_f64_occ(A, h->tile, nt, mh, mode, h->stream)
+                             : launch_stage_p2_f64_occ(A, h->tile, nt, mh, mode, h->stream);
+    return h->cfg.p == 1 ? launch_stage_p1_f64(A, h->tile, nt, mh, mode, h->stream)
+                         : launch_stage_p2_f64(A, h->tile, nt, mh, mode, h->stream);
 }
 cudaError_t launch_stage_any(dgsw_rkdg_s* h, const StageArgs<float>& A, int mode) {
-    const int nt = (int)h->tiling.ntiles, mh = h->tiling.max_halo, me = h->tiling.max_edges;
+    const int nt = (int)h->tiling.ntiles, mh = h->tiling.max_halo;
     if (h->uncapped) mode |= STAGE_MODE_UNCAPPED;
     if (h->split) {
         const int m = mode | (h->occ ? STAGE_MODE_OCC : 0);
-        return h->cfg.p == 1 ? launch_stage_p1_f32_split(A, h->tile, nt, mh, me, m, h->stream)
-                             : launch_stage_p2_f32_split(A, h->tile, nt, mh, me, m, h->stream);
+        return h->cfg.p == 1 ? launch_stage_p1_f32_split(A, h->tile, nt, mh, m, h->stream)
+                             : launch_stage_p2_f32_split(A, h->tile, nt, mh, m, h->stream);
     }
     if (h->occ)
-        return h->cfg.p == 1 ? launch_stage_p1_f32_occ(A, h->tile, nt, mh, me, mode, h->stream)
-                             : launch_stage_p2_f32_occ(A, h->tile, nt, mh, me, mode, h->stream);
-    return h->cfg.p == 1 ? launch_stage_p1_f32(A, h->tile, nt, mh, me, mode, h->stream)
-                         : launch_stage_p2_f32(A, h->tile, nt, mh, me, mode, h->stream);
+        return h->cfg.p == 1 ? launch_stage_p1_f32_occ(A, h->tile, nt, mh, mode, h->stream)
+                             : launch_stage_p2_f32_occ(A, h->tile, nt, mh, mode, h->stream);
+    return h->cfg.p == 1 ? launch_stage_p1_f32(A, h->tile, nt, mh, mode, h->stream)
+                         : launch_stage_p2_f32(A, h->tile, nt, mh, mode, h->stream);
 }
 
 template <typename Real>
@@ -579,6 +575,7 @@ int check_status(dgsw_rkdg_s* h) {
     DevStatus st;
     CUDA_TRY(cudaMemcpyAsync(&st, h->status.p, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
+    if (st.wait_failed) return fail(DGSW_ERR_CUDA, "stage kernel: a barrier wait gave up");
     if (st.nan_flag) {
         // the first stage with a NaN and its smallest element, as the reference's per-stage scrutiny
         // reports it before aborting
@@ -908,20 +905,19 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
     const size_t bath_bytes = (size_t)3 * h->ne_pad * h->real_size;
     if ((e = cudaMalloc(&h->bath, bath_bytes)) != cudaSuccess) return cleanup_fail("bath alloc", e);
     h->device_bytes += bath_bytes;
-    const size_t geo_bytes = (size_t)5 * h->ne_pad * h->real_size;
+    const size_t geo_bytes = (size_t)4 * h->ne_pad * h->real_size;
     if ((e = cudaMalloc(&h->geo, geo_bytes)) != cudaSuccess) return cleanup_fail("geometry alloc", e);
     h->device_bytes += geo_bytes;
-    const size_t n_edges = h->tiling.edges.size() / 4;
-    const size_t egeo_bytes = (size_t)3 * std::max<size_t>(n_edges, 1) * h->real_size;
-    if ((e = cudaMalloc(&h->egeo, egeo_bytes)) != cudaSuccess) return cleanup_fail("edge geometry alloc", e);
-    h->device_bytes += egeo_bytes;
+    const size_t fw_bytes = (size_t)3 * h->ne_pad * h->real_size;
+    if ((e = cudaMalloc(&h->fw, fw_bytes)) != cudaSuccess) return cleanup_fail("face record alloc", e);
+    h->device_bytes += fw_bytes + (size_t)3 * h->ne_pad * sizeof(int);
     // static mesh data in device order
     {
         std::vector<int> en((size_t)3 * h->ne_pad, 0);
         std::vector<double> bathm;
         project_bathymetry(h->topo, h->node_xyz.data(), h->tb, bathm);
         std::vector<double> bdev((size_t)3 * h->ne_pad, 0.0);
-        std::vector<double> gdev((size_t)5 * h->ne_pad, 0.0);
+        std::vector<double> gdev((size_t)4 * h->ne_pad, 0.0);
         std::vector<int> nb((size_t)3 * h->ne_pad, -1);
 #pragma omp parallel for schedule(static)
         for (int64_t d = 0; d < h->ne; ++d) {
@@ -937,16 +933,12 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
             for (int k = 0; k < 3; ++k) bdev[(size_t)k * h->ne_pad + d] = bathm[r * h->nd + k];
             double gg[5];
             element_geometry(h->node_xyz.data(), &h->topo.enodes[3 * r], gg);
-            for (int c = 0; c < 5; ++c) gdev[(size_t)c * h->ne_pad + d] = gg[c];
+            for (int c = 0; c < 4; ++c) gdev[(size_t)c * h->ne_pad + d] = gg[c];
         }
         if ((e = h->enodes.alloc(en.size())) != cudaSuccess) return cleanup_fail("alloc", e);
         cudaMemcpy(h->enodes.p, en.data(), en.size() * sizeof(int), cudaMemcpyHostToDevice);
         if ((e = h->nbr.alloc(nb.size())) != cudaSuccess) return cleanup_fail("alloc", e);
         cudaMemcpy(h->nbr.p, nb.data(), nb.size() * sizeof(int), cudaMemcpyHostToDevice);
-        std::vector<double> edev((size_t)3 * std::max<size_t>(n_edges, 1), 0.0);
-#pragma omp parallel for schedule(static)
-        for (int64_t i = 0; i < (int64_t)n_edges; ++i)
-            for (int c = 0; c < 3; ++c) edev[c * n_edges + i] = h->tiling.egeo[3 * i + c];
         auto upload_real = [&](void* dst, const std::vector<double>& src) {
             if (h->fp32) {
                 std::vector<float> f(src.size());
@@ -959,7 +951,17 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
         };
         upload_real(h->bath, bdev);
         upload_real(h->geo, gdev);
-        upload_real(h->egeo, edev);
+        {
+            std::vector<int> fm((size_t)3 * h->ne_pad, 0);
+            std::vector<double> fw((size_t)3 * h->ne_pad, 0.0);
+            for (int f = 0; f < 3; ++f) {
+                std::copy_n(h->tiling.fmeta.begin() + f * h->ne, h->ne, fm.begin() + (size_t)f * h->ne_pad);
+                std::copy_n(h->tiling.fw.begin() + f * h->ne, h->ne, fw.begin() + (size_t)f * h->ne_pad);
+            }
+            if ((e = h->fmeta.alloc(fm.size())) != cudaSuccess) return cleanup_fail("alloc", e);
+            cudaMemcpy(h->fmeta.p, fm.data(), fm.size() * sizeof(int), cudaMemcpyHostToDevice);
+            upload_real(h->fw, fw);
+        }
         if (cfg->bottom_friction == DGSW_FRICTION_MANNING) {
             std::vector<double> mf, mdev((size_t)h->ne_pad, 0.0);
             manning_factor(h->topo, mesh->node_manning_n, cfg->g, mf);
@@ -1006,9 +1008,8 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
         const size_t nhalo = h->tiling.halo.size() / 2;
         if ((e = h->halo.alloc(std::max<size_t>(nhalo, 1))) != cudaSuccess) return cleanup_fail("alloc", e);
         if (nhalo) cudaMemcpy(h->halo.p, h->tiling.halo.data(), nhalo * sizeof(int2), cudaMemcpyHostToDevice);
-        if ((e = h->tile_halo_off.alloc(h->tiling.tile_halo_off.size())) != cudaSuccess) return cleanup_fail("alloc", e);
-        cudaMemcpy(h->tile_halo_off.p, h->tiling.tile_halo_off.data(), h->tiling.tile_halo_off.size() * sizeof(int),
-                   cudaMemcpyHostToDevice);
+        if ((e = h->tiles.alloc(h->tiling.ntiles)) != cudaSuccess) return cleanup_fail("alloc", e);
+        cudaMemcpy(h->tiles.p, h->tiling.tiles.data(), h->tiling.ntiles * sizeof(int4), cudaMemcpyHostToDevice);
         std::vector<double2> xy(h->nn);
         std::vector<double> nz(h->nn);
         for (int64_t i = 0; i < h->nn; ++i) {
@@ -1019,14 +1020,6 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
         cudaMemcpy(h->xy.p, xy.data(), h->nn * sizeof(double2), cudaMemcpyHostToDevice);
         if ((e = h->nz.alloc(h->nn)) != cudaSuccess) return cleanup_fail("alloc", e);
         cudaMemcpy(h->nz.p, nz.data(), h->nn * sizeof(double), cudaMemcpyHostToDevice);
-        const size_t nedges = n_edges;
-        if ((e = h->edges.alloc(std::max<size_t>(nedges, 1))) != cudaSuccess) return cleanup_fail("alloc", e);
-        if (nedges) cudaMemcpy(h->edges.p, h->tiling.edges.data(), nedges * sizeof(int4), cudaMemcpyHostToDevice);
-        if ((e = h->tile_edge_off.alloc(h->tiling.tile_edge_off.size())) != cudaSuccess) return cleanup_fail("alloc", e);
-        cudaMemcpy(h->tile_edge_off.p, h->tiling.tile_edge_off.data(), h->tiling.tile_edge_off.size() * sizeof(int),
-                   cudaMemcpyHostToDevice);
-        if ((e = h->eslot.alloc(h->ne)) != cudaSuccess) return cleanup_fail("alloc", e);
-        cudaMemcpy(h->eslot.p, h->tiling.eslot.data(), h->ne * sizeof(int2), cudaMemcpyHostToDevice);
         if ((e = h->ref_of_dev.alloc(h->ne)) != cudaSuccess) return cleanup_fail("alloc", e);
         cudaMemcpy(h->ref_of_dev.p, h->tiling.ref_of_dev.data(), h->ne * sizeof(int), cudaMemcpyHostToDevice);
         for (int i = 0; i < 2; ++i) {
@@ -1070,7 +1063,7 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
             if ((e = h->l2rule.alloc(1)) != cudaSuccess) return cleanup_fail("alloc", e);
             cudaMemcpy(h->l2rule.p, &Rh, sizeof(L2Rule), cudaMemcpyHostToDevice);
         }
-        h->device_bytes += en.size() * 4 + nb.size() * 4 + h->nn * 24 + nedges * 16 + h->ne * 12 + 3 * h->ne_pad;
+        h->device_bytes += en.size() * 4 + nb.size() * 4 + h->nn * 24 + h->tiling.ntiles * 16 + nhalo * 8 + h->ne * 4 + 3 * h->ne_pad;
     }
     if (cfg->slope_limiting) {
         // the limiter's geometry, once (the same device code the limiter would run per stage)
@@ -1249,7 +1242,7 @@ static int32_t create_tuned(const dgsw_config* cfg, const dgsw_mesh* mesh, const
         // faster kept. Measured per step: sized to the mesh, config 2 runs 1.5 % (FP32) and 4.9 % (FP64)
         // faster and the p = 2 tidal channel 6.9 % (FP64); the p = 1 bowl stays capped (7 % slower sized).
         chosen.uncapped = 0;
-        if (stage_fits_caps(best->tile, best->tiling.max_halo, best->tiling.max_edges)) {
+        if (stage_fits_caps(best->tile, best->tiling.max_halo)) {
             double t[2] = {0.0, 0.0};
             bool ok = true;
             for (int round = 0; round < 3 && ok; ++round)
@@ -1495,7 +1488,8 @@ int32_t dgsw_rkdg_destroy(dgsw_handle h) {
         if (p) cudaFree(p);
     if (h->bath) cudaFree(h->bath);
     if (h->geo) cudaFree(h->geo);
-    if (h->egeo) cudaFree(h->egeo);
+    h->fmeta.release();
+    if (h->fw) cudaFree(h->fw);
     if (h->manning) cudaFree(h->manning);
     h->fface.release();
     h->fcon.release();
@@ -1506,12 +1500,9 @@ int32_t dgsw_rkdg_destroy(dgsw_handle h) {
     h->post.release();
     h->post_flags.release();
     h->halo.release();
-    h->tile_halo_off.release();
+    h->tiles.release();
     h->enodes.release();
-    h->tile_edge_off.release();
     h->ref_of_dev.release();
-    h->eslot.release();
-    h->edges.release();
     h->xy.release();
     h->nz.release();
     h->wet[0].release();
@@ -1554,7 +1545,7 @@ int32_t dgsw_rkdg_info(dgsw_handle h, dgsw_info* o) {
     o->n_interfaces = (int64_t)h->topo.intf.size() / 4;
     o->n_boundaries = (int64_t)h->topo.bnd.size() / 3;
     o->n_tiles = h->tiling.ntiles;
-    o->n_tile_edges = (int64_t)h->tiling.edges.size() / 4;
+    o->n_tile_edges = h->tiling.n_edges;
     o->p = h->cfg.p;
     o->ndof = h->nd;
     o->ngp_volume = h->tb.nq;
@@ -1567,7 +1558,7 @@ int32_t dgsw_rkdg_info(dgsw_handle h, dgsw_info* o) {
     o->occupancy = h->occ;
     o->tile_order = h->order;
     o->stage_increments = h->split ? 1 : 0;
-    o->smem_capped = (!h->uncapped && stage_fits_caps(h->tile, h->tiling.max_halo, h->tiling.max_edges)) ? 1 : 0;
+    o->smem_capped = (!h->uncapped && stage_fits_caps(h->tile, h->tiling.max_halo)) ? 1 : 0;
     return DGSW_OK;
 }
 

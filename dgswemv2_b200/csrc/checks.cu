@@ -20,7 +20,7 @@ namespace {
 
 using dgsw::Flux2;
 
-// the interface Gauss point of the stage kernel's phase 2 for an internal edge: LLF with sp on the in
+// the interface Gauss point of the stage kernel's face loop: LLF (llf_sides, or llf_flux where sp differs from 1) with sp on the in
 // side, F_ex = -F_in, and the wet/dry fix-ups when either side is dry (rkdg_swe_is_internal.hpp:26-95)
 template <typename Real>
 __global__ void check_flux_kernel(int n, Real g, const double* __restrict__ qin, const double* __restrict__ qex,
@@ -34,7 +34,19 @@ __global__ void check_flux_kernel(int n, Real g, const double* __restrict__ qin,
     const Real qe[3] = {(Real)qex[3 * i], (Real)qex[3 * i + 1], (Real)qex[3 * i + 2]};
     const Real nx = (Real)nrm[2 * i], ny = (Real)nrm[2 * i + 1];
     Real F[3];
-    dgsw::llf_flux<Real>(g, qi, qe, (Real)bin[i], (Real)sp[i], nx, ny, F);
+    if ((Real)sp[i] == Real(1)) {
+        // the face loop's form: both sides on the in side's bathymetry, a unit normal, the doubled flux
+        dgsw::Side<Real> a, b;
+        a.q = {qi[1], qi[2]}, a.ze = qi[0], a.b = (Real)bin[i];
+        b.q = {qe[1], qe[2]}, b.ze = qe[0], b.b = (Real)bin[i];
+        dgsw::complete<Real>(a, g);
+        dgsw::complete<Real>(b, g);
+        dgsw::Two<Real> F12;
+        dgsw::llf_sides<sizeof(Real) == 4, Real>(g, a, b, dgsw::Two<Real>{nx, ny}, Real(1), F[0], F12);
+        F[0] *= Real(0.5), F[1] = Real(0.5) * F12.x, F[2] = Real(0.5) * F12.y;
+    } else {
+        dgsw::llf_flux<Real>(g, qi, qe, (Real)bin[i], (Real)sp[i], nx, ny, F);
+    }
     Real E[3] = {-F[0], -F[1], -F[2]};
     if (internal) {
         const bool wa = wet_in[i] != 0, wb = wet_ex[i] != 0;

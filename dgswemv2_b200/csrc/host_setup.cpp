@@ -504,34 +504,6 @@ void face_geometry(const double* X, const int32_t* nd, int f, double& nx, double
     sJ = std::sqrt(std::pow(dx, 2.0) + std::pow(dy, 2.0)) / 2.0;
 }
 
-// open-addressing map from non-negative keys to small ints, for the per-tile edge and halo lookups (a few
-// hundred entries per tile); clear() forgets only the slots in use
-struct FlatMap {
-    static constexpr int CAP = 4096;  // > 2 x the largest tile list (1022 edges, 3 x 256 + halo faces)
-    std::vector<int64_t> keys = std::vector<int64_t>(CAP, -1);
-    std::vector<int32_t> vals = std::vector<int32_t>(CAP, 0);
-    std::vector<int32_t> used;
-    static uint32_t slot(int64_t k) { return (uint32_t)(((uint64_t)k * 0x9E3779B97F4A7C15ull) >> 52) & (CAP - 1); }
-    int find(int64_t k) const {
-        for (uint32_t i = slot(k);; i = (i + 1) & (CAP - 1)) {
-            if (keys[i] == k) return vals[i];
-            if (keys[i] < 0) return -1;
-        }
-    }
-    void insert(int64_t k, int32_t v) {
-        uint32_t i = slot(k);
-        while (keys[i] >= 0) i = (i + 1) & (CAP - 1);
-        keys[i] = k;
-        vals[i] = v;
-        used.push_back((int32_t)i);
-    }
-    int size() const { return (int)used.size(); }
-    void clear() {
-        for (int32_t i : used) keys[i] = -1;
-        used.clear();
-    }
-};
-
 int build_tiling(const Topology& T, const double* X, int tile, bool morton, Tiling& out, std::string& err) {
     const int64_t ne = T.ne;
     if (tile != 64 && tile != 128 && tile != 256) {
@@ -579,13 +551,11 @@ int build_tiling(const Topology& T, const double* X, int tile, bool morton, Tili
     out.dev_of_ref.resize(ne);
     for (int64_t d = 0; d < ne; ++d) out.dev_of_ref[out.ref_of_dev[d]] = (int32_t)d;
     out.ntiles = (ne + tile - 1) / tile;
-    out.tile_edge_off.assign(out.ntiles + 1, 0);
-    out.tile_halo_off.assign(out.ntiles + 1, 0);
-    out.edges.clear();
-    out.egeo.clear();
+    out.tiles.assign((size_t)4 * out.ntiles, 0);
+    out.fmeta.resize((size_t)3 * ne);
+    out.fw.resize((size_t)3 * ne);
     out.halo.clear();
-    out.eslot.assign(2 * ne, 0);
-    out.max_edges = 0;
+    out.n_edges = 0;
     out.max_halo = 0;
     std::vector<int32_t> iface(3 * ne, -1);
     const int64_t n_intf = (int64_t)T.intf.size() / 4;
@@ -596,133 +566,88 @@ int build_tiling(const Topology& T, const double* X, int tile, bool morton, Tili
     }
     std::vector<int32_t> bface(3 * ne, -1);
     for (size_t i = 0; i < T.bnd.size() / 3; ++i) bface[3 * (int64_t)T.bnd[3 * i] + T.bnd[3 * i + 1]] = (int32_t)i;
-    // tiles are independent: each builds its own edge, geometry and halo lists (in parallel), and the
-    // lists are concatenated in tile order
-    struct TileLists {
-        std::vector<int32_t> te;  // edge records
-        std::vector<double> tg;   // edge geometry
-        std::vector<int32_t> halo;
-    };
-    std::vector<TileLists> lists((size_t)out.ntiles);
-    int overflow = 0;
-#pragma omp parallel
-    {
-        FlatMap local_edge, local_halo;
-#pragma omp for schedule(dynamic, 16) reduction(| : overflow)
-        for (int64_t t = 0; t < out.ntiles; ++t) {
-            local_edge.clear();
-            local_halo.clear();
-            std::vector<int32_t>& te = lists[t].te;
-            te.reserve(4 * (size_t)(3 * tile / 2 + 32));
-            std::vector<double>& tg = lists[t].tg;
-            std::vector<int32_t>& halo = lists[t].halo;
-            const int64_t d0 = t * tile, d1 = std::min(ne, d0 + tile);
-            // trace slot of (element in reference order, face)
-            auto trace_slot = [&](int32_t r, int f) -> int32_t {
-                const int64_t d = out.dev_of_ref[r];
-                if (d >= d0 && d < d1) return (int32_t)(3 * (d - d0) + f);
-                const int64_t key = 3 * (int64_t)r + f;
-                const int found = local_halo.find(key);
-                if (found >= 0) return 3 * tile + found;
-                const int h = local_halo.size();
-                local_halo.insert(key, h);
-                halo.push_back((int32_t)d);
-                halo.push_back(f);
-                return 3 * tile + h;
-            };
-            for (int64_t d = d0; d < d1; ++d) {
-                const int32_t r = out.ref_of_dev[d];
-                uint32_t slots[3] = {1023, 1023, 1023};
-                for (int f = 0; f < 3; ++f) {
-                    const int64_t ii = iface[3 * (int64_t)r + f];
-                    const int64_t bi = bface[3 * (int64_t)r + f];
-                    if (ii >= 0) {
-                        const int found = local_edge.find(ii);
-                        if (found >= 0) {
-                            slots[f] = (uint32_t)found;
-                            continue;
+    // tiles are independent: each writes its elements' face records and builds its own list (in parallel), and
+    // the lists are concatenated in tile order
+    std::vector<std::vector<int32_t>> lists((size_t)out.ntiles);
+    int64_t n_edges = 0;
+#pragma omp parallel for schedule(dynamic, 16) reduction(+ : n_edges)
+    for (int64_t t = 0; t < out.ntiles; ++t) {
+        std::vector<int32_t>& halo = lists[t];
+        std::vector<int32_t> boundary;  // device element, face
+        const int64_t d0 = t * tile, d1 = std::min(ne, d0 + tile);
+        for (int64_t d = d0; d < d1; ++d) {
+            const int32_t r = out.ref_of_dev[d];
+            double J[5];
+            element_geometry(X, &T.enodes[3 * (int64_t)r], J);
+            for (int f = 0; f < 3; ++f) {
+                const int64_t ii = iface[3 * (int64_t)r + f];
+                const int64_t bi = bface[3 * (int64_t)r + f];
+                const int32_t own = (int32_t)(3 * (d - d0) + f);
+                double nx = 0.0, ny = 0.0, sJ = 0.0;
+                int32_t meta = EK_NONE | 1 << 3 | own << 4;
+                if (ii >= 0) {
+                    const bool in = T.intf[4 * ii] == r && T.intf[4 * ii + 2] == f;
+                    face_geometry(X, &T.enodes[3 * (int64_t)T.intf[4 * ii]], T.intf[4 * ii + 2], nx, ny, sJ);
+                    const int32_t other = T.intf[4 * ii + (in ? 1 : 0)], of = T.intf[4 * ii + (in ? 3 : 2)];
+                    const int64_t od = out.dev_of_ref[other];
+                    const bool here = od >= d0 && od < d1;
+                    if (!here || od > d) ++n_edges;
+                    if (ii >= T.n_intf_internal) {
+                        meta = EK_LEVEE | (in ? 1 : 0) << 3 | (int32_t)(ii - T.n_intf_internal) << 4;
+                    } else {
+                        int32_t slot = (int32_t)(3 * (od - d0)) + of;
+                        if (!here) {
+                            slot = 3 * tile + (int32_t)(halo.size() / 2);
+                            halo.push_back((int32_t)od);
+                            halo.push_back(of);
                         }
-                        const int idx = (int)(te.size() / 4);
-                        local_edge.insert(ii, idx);
-                        slots[f] = (uint32_t)idx;
-                        const int32_t in = T.intf[4 * ii], ex = T.intf[4 * ii + 1];
-                        const int fin = T.intf[4 * ii + 2], fex = T.intf[4 * ii + 3];
-                        te.push_back(trace_slot(in, fin));
-                        te.push_back(trace_slot(ex, fex));
-                        // levee interfaces carry their index among the levee interfaces above bit 8
-                        const bool lev = ii >= T.n_intf_internal;
-                        te.push_back(lev ? (fin | fex << 2 | EK_LEVEE << 4 | (int32_t)(ii - T.n_intf_internal) << 8)
-                                         : (fin | fex << 2 | EK_INTERIOR << 4));
-                        te.push_back(out.dev_of_ref[in]);
-                        double nx, ny, sJ;
-                        face_geometry(X, &T.enodes[3 * (int64_t)in], fin, nx, ny, sJ);
-                        tg.push_back(nx);
-                        tg.push_back(ny);
-                        tg.push_back(sJ);
-                    } else if (bi >= 0) {
-                        const int idx = (int)(te.size() / 4);
-                        slots[f] = (uint32_t)idx;
-                        const int bt = T.bnd[3 * bi + 2];
-                        const int kind = bt == DGSW_BC_LAND   ? EK_LAND
-                                         : bt == DGSW_BC_TIDE ? EK_TIDE
-                                         : bt == DGSW_BC_FLOW ? EK_FLOW
-                                                              : EK_FUNCTION;
-                        // tide / flow faces carry their forcing record as -2 - index in the b slot
-                        const int32_t fidx = (kind == EK_TIDE || kind == EK_FLOW) ? T.bnd_force[bi] : -1;
-                        te.push_back((int32_t)(3 * (d - d0) + f));
-                        te.push_back(fidx >= 0 ? -2 - fidx : -1);
-                        te.push_back(f | kind << 4);
-                        te.push_back((int32_t)d);
-                        double nx, ny, sJ;
-                        face_geometry(X, &T.enodes[3 * (int64_t)r], f, nx, ny, sJ);
-                        tg.push_back(nx);
-                        tg.push_back(ny);
-                        tg.push_back(sJ);
+                        meta = EK_INTERIOR | (in ? 1 : 0) << 3 | slot << 4;
                     }
+                } else if (bi >= 0) {
+                    face_geometry(X, &T.enodes[3 * (int64_t)r], f, nx, ny, sJ);
+                    boundary.push_back((int32_t)d);
+                    boundary.push_back(f);
+                    ++n_edges;
                 }
-                int32_t roles = 0;
-                for (int f = 0; f < 3; ++f) roles |= (T.is_in[3 * r + f] ? 1 : 0) << f;
-                int32_t ord = T.order_count[r];
-                for (int k = 0; k < T.order_count[r]; ++k) ord |= T.order_face[3 * r + k] << (2 + 2 * k);
-                out.eslot[2 * d] = (int32_t)(slots[0] | slots[1] << 10 | slots[2] << 20);
-                out.eslot[2 * d + 1] = roles | ord << 3;
+                const int64_t at = f * ne + d;
+                out.fmeta[at] = meta;
+                out.fw[at] = sJ / J[4];
             }
-            if (te.size() / 4 > 1022) overflow = 1;
+        }
+        out.tiles[4 * t + 1] = (int32_t)(halo.size() / 2);
+        // boundary faces after the halo faces: tide / flow faces carry their forcing record
+        for (size_t k = 0; k < boundary.size(); k += 2) {
+            const int32_t d = boundary[k], f = boundary[k + 1];
+            const int64_t bi = bface[3 * (int64_t)out.ref_of_dev[d] + f];
+            const int bt = T.bnd[3 * bi + 2];
+            const int kind = bt == DGSW_BC_LAND   ? EK_LAND
+                             : bt == DGSW_BC_TIDE ? EK_TIDE
+                             : bt == DGSW_BC_FLOW ? EK_FLOW
+                                                  : EK_FUNCTION;
+            out.fmeta[f * ne + d] = kind | 1 << 3 | (3 * tile + (int32_t)(halo.size() / 2)) << 4;
+            halo.push_back(kind == EK_TIDE || kind == EK_FLOW ? T.bnd_force[bi] : -1);
+            halo.push_back(0);
+        }
+        out.tiles[4 * t + 2] = (int32_t)(halo.size() / 2);
+    }
+    out.n_edges = n_edges;
+    // offsets by a prefix sum over the tiles, then every tile copies its list into place
+    int64_t total = 0;
+    for (int64_t t = 0; t < out.ntiles; ++t) {
+        out.tiles[4 * t] = (int32_t)total;
+        total += (int64_t)lists[t].size() / 2;
+        out.max_halo = std::max(out.max_halo, (int)(lists[t].size() / 2));
+        if (total >= std::numeric_limits<int32_t>::max()) {
+            err = "too many halo faces";
+            return DGSW_ERR_UNSUPPORTED;
         }
     }
-    if (overflow) {
-        err = "tile edge list overflow";
-        return DGSW_ERR_INVALID_ARGUMENT;
-    }
-    // offsets by a prefix sum over the tiles, then every tile copies its lists into place
-    std::vector<int64_t> eo(out.ntiles + 1, 0), ho(out.ntiles + 1, 0);
-    for (int64_t t = 0; t < out.ntiles; ++t) {
-        eo[t + 1] = eo[t] + (int64_t)lists[t].te.size() / 4;
-        ho[t + 1] = ho[t] + (int64_t)lists[t].halo.size() / 2;
-        out.max_edges = std::max(out.max_edges, (int)(lists[t].te.size() / 4));
-        out.max_halo = std::max(out.max_halo, (int)(lists[t].halo.size() / 2));
-    }
-    if (eo[out.ntiles] >= std::numeric_limits<int32_t>::max() || ho[out.ntiles] >= std::numeric_limits<int32_t>::max()) {
-        err = "too many tile edges";
-        return DGSW_ERR_UNSUPPORTED;
-    }
-    out.edges.resize((size_t)4 * eo[out.ntiles]);
-    out.egeo.resize((size_t)3 * eo[out.ntiles]);
-    out.halo.resize((size_t)2 * ho[out.ntiles]);
+    out.halo.resize((size_t)2 * total);
 #pragma omp parallel for schedule(dynamic, 64)
     for (int64_t t = 0; t < out.ntiles; ++t) {
-        TileLists& L = lists[t];
-        out.tile_edge_off[t] = (int32_t)eo[t];
-        out.tile_halo_off[t] = (int32_t)ho[t];
-        std::copy(L.te.begin(), L.te.end(), out.edges.begin() + 4 * eo[t]);
-        std::copy(L.tg.begin(), L.tg.end(), out.egeo.begin() + 3 * eo[t]);
-        std::copy(L.halo.begin(), L.halo.end(), out.halo.begin() + 2 * ho[t]);
-        std::vector<int32_t>().swap(L.te);
-        std::vector<double>().swap(L.tg);
-        std::vector<int32_t>().swap(L.halo);
+        std::copy(lists[t].begin(), lists[t].end(), out.halo.begin() + 2 * (int64_t)out.tiles[4 * t]);
+        std::vector<int32_t>().swap(lists[t]);
     }
-    out.tile_edge_off[out.ntiles] = (int32_t)((int64_t)out.edges.size() / 4);
-    out.tile_halo_off[out.ntiles] = (int32_t)((int64_t)out.halo.size() / 2);
     return DGSW_OK;
 }
 

@@ -41,8 +41,8 @@ constexpr int MAX_ND = 6;  // p <= 2
 constexpr int MAX_NQ = 6;
 constexpr int MAX_NG = 3;
 
-// Edge kinds in the per-tile edge lists
-enum EdgeKind { EK_INTERIOR = 0, EK_LAND = 1, EK_FUNCTION = 2, EK_TIDE = 3, EK_FLOW = 4, EK_LEVEE = 5 };
+// Kinds of an element's face; EK_NONE: a face without a boundary object (outflow, an unpaired levee face)
+enum EdgeKind { EK_INTERIOR = 0, EK_LAND = 1, EK_FUNCTION = 2, EK_TIDE = 3, EK_FLOW = 4, EK_LEVEE = 5, EK_NONE = 7 };
 
 struct Topology {
     int64_t ne = 0, nn = 0;
@@ -102,17 +102,17 @@ struct Tiling {
     int64_t ntiles = 0;
     std::vector<int32_t> dev_of_ref;  // [ne]
     std::vector<int32_t> ref_of_dev;  // [ne]
-    std::vector<int32_t> tile_edge_off;  // [ntiles+1]
-    // [4 * n_edges]: trace slot of the in/owner side a, trace slot of b (-1 for boundaries),
-    // meta = face_a | face_b << 2 | kind << 4, device index of a. Trace slots: 3*(element - tile start)
-    // + face for tile elements, 3*tile + h for the tile's halo face h.
-    bigvec<int32_t> edges;
-    bigvec<double> egeo;                 // [3 * n_edges]: normal x, normal y, half length (of face a)
-    std::vector<int32_t> tile_halo_off;  // [ntiles+1]
-    bigvec<int32_t> halo;                // [2 * n_halo]: device element, face
-    std::vector<int32_t> eslot;          // [2 * ne] per element (dev order): packed slots, roles + order
-    int max_edges = 0;
-    int max_halo = 0;
+    // per face f of device element d, at [f * ne + d]: kind | (the element is the interface's in side) << 3 |
+    // payload << 4, the payload being the trace slot across the face (a levee interface: its index among them).
+    // Trace slots: 3*(element - tile start) + face for tile elements, 3*tile + h for entry h of the tile's list.
+    bigvec<int32_t> fmeta;
+    bigvec<double> fw;                   // [3 * ne] half the face's length over the element's |J|
+    // per tile: offset into halo, halo faces, halo + boundary faces, 0
+    std::vector<int32_t> tiles;          // [4 * ntiles]
+    // [2 * n]: per tile its halo faces (device element, face), then its boundary faces (forcing record or -1, 0)
+    bigvec<int32_t> halo;
+    int64_t n_edges = 0;                 // edges of all tiles (one between two tiles counts for both)
+    int max_halo = 0;                    // most halo and boundary faces of a tile
 };
 
 int build_tiling(const Topology& T, const double* node_xyz, int tile, bool morton, Tiling& out, std::string& err);

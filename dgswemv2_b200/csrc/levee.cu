@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(128) levee_kernel(const LeveeArgs<Real> A) {
         llf_flux<double>(g_ex, qe, q_ex_ex, te[3][ge], D[2 + 12 + ge], -nx, -ny, Fe);
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
-            F[v * NG + g] = Fi[v];
-            F[(3 + v) * NG + g] = Fe[v];
+            F[v * NG + g] = wet_in || wet_ex ? Fi[v] : 0.0;  // both sides dry: no exchange
+            F[(3 + v) * NG + g] = wet_in || wet_ex ? Fe[v] : 0.0;
         }
     }
 }

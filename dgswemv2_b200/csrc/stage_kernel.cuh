@@ -1,21 +1,28 @@
 // Fused RKDG stage kernel for sm_100a.
 //
 // One CTA owns one tile of TILE consecutive elements (device order = Morton order of centroids).
-// Per RK stage it does, in three phases separated by __syncthreads:
-//   1. element phase (thread = element): load the element's modes, accumulate the volume and source
-//      integrals in registers (Problem::volume_kernel + source_kernel, rkdg_swe_proc_volume.hpp:9-35,
-//      rkdg_swe_proc_source.hpp:9-18), and write the traces of its three faces at the edge Gauss points
-//      to shared memory. Neighbours in other tiles ("halo" faces) get their face traces written by the
-//      same routine from global memory;
-//   2. edge phase (thread = edge of the tile's list): numerical flux at the edge Gauss points once per
-//      edge from the shared-memory traces (interfaces: LLF + the wet/dry fix-ups of ISP::Internal,
-//      rkdg_swe_is_internal.hpp:26-95; boundaries: BC::Land / BC::Function, rkdg_swe_bc_land.hpp:41-66,
-//      rkdg_swe_bc_function.hpp:27-60). An edge between two tiles is evaluated by both CTAs with the
-//      same code on the same bits, so F_ex = -F_in holds exactly as in the reference;
-//   3. element phase: subtract the edge contributions in the reference's interface/boundary order,
-//      apply M^-1 and the SSP-RK stage combination (element.hpp:502-505,
-//      explicit_ssp_rk_stepper.hpp:67-80), the wetting/drying kernel (swe_post_wet_dry.hpp:6-145, its
-//      depth tests in FP64 in every precision) and the NaN scrutiny; write the next stage state.
+// Per RK stage it does, thread = element:
+//   1. loads the element's modes and writes the traces of its three faces at the edge Gauss points to shared
+//      memory. Neighbours in other tiles ("halo" faces) get their face traces written by the same routine
+//      from global memory, and a boundary face's ghost state (BC::Land / Tide / Flow / Function,
+//      rkdg_swe_bc_land.hpp:41-66, rkdg_swe_bc_function.hpp:27-60) goes to a trace slot of its own, so that the
+//      face loop below has no boundary branches. Then the thread arrives on the CTA's one barrier;
+//   2. accumulates the volume and source integrals in registers (Problem::volume_kernel + source_kernel,
+//      rkdg_swe_proc_volume.hpp:9-35, rkdg_swe_proc_source.hpp:9-18) while the other warps' traces arrive;
+//   3. waits on the barrier and takes the numerical flux of its own three faces (LLF + the wet/dry fix-ups of
+//      ISP::Internal, rkdg_swe_is_internal.hpp:26-95) straight into the lift. Both elements of an interface
+//      evaluate the flux, each with its outward normal; the formula is arranged so that the two are exact
+//      negatives of each other, as in the reference;
+//   4. applies M^-1 and the SSP-RK stage combination (element.hpp:502-505,
+//      explicit_ssp_rk_stepper.hpp:67-80), the wetting/drying kernel (swe_post_wet_dry.hpp:6-145, its depth
+//      tests in FP64 in every precision) and the NaN scrutiny; writes the next stage state.
+// What bounds it: latency and instruction issue, not bytes (20-35 % of the HBM rate), so it is arranged for few
+// instructions and few waits. Evaluating each flux twice costs about four more LLF evaluations per element than
+// one per edge of the tile, and saves the flux's way through shared memory, the edge lists, a second barrier and the
+// half-empty second round of edges. Against one flux per edge between two barriers, 524,288 triangles, p = 2, FP32:
+// warp instructions of the second stage 46.7 M -> 33.9 M, barrier stalls 1.3 -> 0.1 per issue, cold 97.7 -> 77.9 us;
+// 8 steps 2.36 -> 1.95 ms (FP64 4.74 -> 4.18 ms); tidal channel p = 1 of 433,394 FP32 0.74 -> 0.56 ms; ensemble of 24
+// wet/dry members FP32 1.84 -> 1.42 ms.
 // The master tables are compile-time constants (tables_gen.h): every table entry is an immediate,
 // zero entries are skipped and unit entries become additions.
 // HBM layout: component-major SoA, q[(var*ND + dof) * ne_pad + element].
@@ -23,6 +30,7 @@
 #define DGSW_STAGE_KERNEL_CUH
 
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/dgsw_rkdg.h"
 #include "function_sets.h"
@@ -35,6 +43,7 @@ namespace dgsw {
 template <int N>
 struct IC {
     static constexpr int value = N;
+    __device__ constexpr operator int() const { return N; }
 };
 template <int B, int E, typename F>
 __device__ __forceinline__ void sfor(F&& f) {
@@ -44,22 +53,61 @@ __device__ __forceinline__ void sfor(F&& f) {
     }
 }
 
-// packed FP32 arithmetic of sm_100 (one FFMA2 issue for two FMAs): a0 += x0 c0 and a1 += x1 c1. Each lane is
-// an IEEE fma with the scalar fma's rounding. The kernels pair variables (ze with qx; qy with the bathymetry
-// or alone) so that both lanes share one coefficient. Z0 / Z1 mark terms whose coefficient is a compile-time
-// zero; they are left out, as the scalar loops leave them out.
-template <bool Z0 = false, bool Z1 = false>
-__device__ __forceinline__ void fma_pair(float& a0, float& a1, float x0, float x1, float c0, float c1) {
-    if constexpr (!Z0 && !Z1) {
-        const float2 r = __ffma2_rn(make_float2(x0, x1), make_float2(c0, c1), make_float2(a0, a1));
-        a0 = r.x;
-        a1 = r.y;
-    } else if constexpr (!Z0) {
-        a0 = __fmaf_rn(x0, c0, a0);
-    } else if constexpr (!Z1) {
-        a1 = __fmaf_rn(x1, c1, a1);
+// explicitly rounded operations: the two sides of an interface evaluate the flux from either side, and the
+// compiler's choice of contractions must not differ between the own and the neighbour term
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// Two values of one kind, (qx, qy) or (ze, b). PK: one packed FP32 instruction of sm_100 for both
+// (FFMA2 / FMUL2 / FADD2, each lane an IEEE operation); otherwise two scalar ones. The pairs are those that a
+// trace vector holds side by side, so that no register moves are needed to form them.
+template <typename Real>
+struct Two {
+    Real x, y;
+};
+template <bool PK, typename Real>
+__device__ __forceinline__ Two<Real> fma2(Two<Real> a, Two<Real> b, Two<Real> c) {
+    if constexpr (PK) {
+        const float2 r = __ffma2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y), make_float2(c.x, c.y));
+        return {r.x, r.y};
+    } else {
+        return {fma_rn(a.x, b.x, c.x), fma_rn(a.y, b.y, c.y)};
     }
 }
+template <bool PK, typename Real>
+__device__ __forceinline__ Two<Real> fma2(Two<Real> a, Real b, Two<Real> c) {
+    return fma2<PK, Real>(a, Two<Real>{b, b}, c);
+}
+template <bool PK, typename Real>
+__device__ __forceinline__ Two<Real> mul2(Two<Real> a, Two<Real> b) {
+    if constexpr (PK) {
+        const float2 r = __fmul2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+        return {r.x, r.y};
+    } else {
+        return {mul_rn(a.x, b.x), mul_rn(a.y, b.y)};
+    }
+}
+template <bool PK, typename Real>
+__device__ __forceinline__ Two<Real> mul2(Two<Real> a, Real b) {
+    return mul2<PK, Real>(a, Two<Real>{b, b});
+}
+template <bool PK, typename Real>
+__device__ __forceinline__ Two<Real> add2(Two<Real> a, Two<Real> b) {
+    if constexpr (PK) {
+        const float2 r = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+        return {r.x, r.y};
+    } else {
+        return {add_rn(a.x, b.x), add_rn(a.y, b.y)};
+    }
+}
+
+// whether a table entry counts: the quadrature points are rounded, so entries that are zero in exact
+// arithmetic come out as a few 1e-16 of the table's entries near 1
+constexpr bool counts(double c) { return c > 1e-13 || c < -1e-13; }
 
 // NaN scrutiny (scrutinize_solution after every stage, rkdg_swe_proc_serial_step.hpp:59-65): the reference
 // stops at the first stage whose state holds a NaN and reports the first element (ascending ID) there.
@@ -68,13 +116,17 @@ __device__ __forceinline__ void fma_pair(float& a0, float& a1, float x0, float x
 struct DevStatus {
     unsigned long long nan_key;  // ~0 while no NaN has been seen
     unsigned int nan_flag;
-    unsigned int pad;
+    unsigned int wait_failed;  // a CTA gave up waiting at its barrier
 };
+
+constexpr int SINE_NCONST = 10;
 
 // What a stage needs of its time (t + dt drk[s]): the function set's time factors and the forcing ramp
 struct StageTime {
     dgsw_fn_time ft;
     double ramp;
+    double sine[SINE_NCONST];  // the manufactured sine set's constants (SineSrc), in both precisions
+    float sine_f[SINE_NCONST];
 };
 
 struct DevClock {
@@ -112,6 +164,21 @@ struct TimeArgs {
     double* fval;  // [nsets][n_forced][ng] written for `next`
 };
 
+// The manufactured sine set at one stage time: ze = c1 P, qx = -c2 Q, qy = c2 R, zex = c3 Q, zey = -c3 R,
+// zet = -c4 P, qxx = qyy = c5 P, qxy = qyx = c5 S, qxt = -c6 Q, qyt = c6 R with P = sx cy, Q = cx cy, R = sx sy,
+// S = cx sy; c0 = 2 c5 - c4 is the continuity source's. {k, c1, c2, c3, c5, c6, c0, g, H, k / pi}
+__device__ __forceinline__ void sine_constants(const double* P, StageTime& S) {
+    const double k = 2.0 * M_PI / P[0], A = P[1], w = S.ft.s[2], B = P[1] * S.ft.s[2] / (2.0 * k);
+    const double st = S.ft.s[0], ct = S.ft.s[1];
+    const double c[SINE_NCONST] = {k,      A * ct, B * st, A * k * ct, B * k * st, B * w * ct, 2.0 * B * k * st - A * w * st,
+                                   P[4],   P[2],   2.0 / P[0]};
+#pragma unroll
+    for (int i = 0; i < SINE_NCONST; ++i) {
+        S.sine[i] = c[i];
+        S.sine_f[i] = (float)c[i];
+    }
+}
+
 // the ramp of ESSPRKStepper::operator++, explicit_ssp_rk_stepper.hpp:49-65 (1 without a ramp)
 __device__ __forceinline__ double forcing_ramp(const TimeArgs& T, double t) {
     return T.ramp_on ? tanh(2.0 * (t / 86400.0) / T.ramp_duration) : 1.0;
@@ -129,6 +196,7 @@ static __device__ __noinline__ void form_step_time(const TimeArgs* Tp, int block
         if (s < T.nstages) {
             T.next->at[s].ft = dgsw_fn_prepare(T.fn_set, T.fn_params, t + T.off[s]);
             T.next->at[s].ramp = forcing_ramp(T, t + T.off[s]);
+            if (T.fn_set == DGSW_FN_MANUFACTURED_SINE) sine_constants(T.fn_params, T.next->at[s]);
         }
         if (s == 0) {
             T.next->t = t;
@@ -169,14 +237,14 @@ struct StageArgs {
     double* q_out;
     double* sol_out;
     const Real* bath;           // [3][ne_pad] bathymetry modes of the linear part
-    const Real* geo;            // [5][ne_pad] J^-1(0,0), J^-1(0,1), J^-1(1,0), J^-1(1,1), |J|
+    const Real* geo;            // [4][ne_pad] J^-1(0,0), J^-1(0,1), J^-1(1,0), J^-1(1,1)
     const int* enodes;          // [3][ne_pad]
-    const int2* eslot;          // [ne] edge slot per face, roles, accumulation order
-    const int4* edges;          // tile edge lists: trace slot of a, trace slot of b (-1), meta, element a
-    const Real* egeo;           // [3][n_edges]: outward unit normal of a (x, y), half length
-    const int* tile_edge_off;
-    const int2* halo;           // tile halo lists: (element, face)
-    const int* tile_halo_off;
+    // per face: kind (bits 0-2, EdgeKind) | the element is the interface's in side (bit 3) | payload << 4: the trace
+    // slot across the face (a neighbour's, or the boundary face's ghost slot), or the levee interface's index
+    const int* fmeta;           // [3][ne_pad]
+    const Real* fw;             // [3][ne_pad] half the face's length over the element's |J|
+    const int4* tiles;          // per tile: offset into halo, halo faces, halo + boundary faces
+    const int2* halo;           // tile lists: (element, face) per halo face, then (forcing record, 0) per boundary face
     const double2* xy;          // node coordinates
     const double* nz;           // node bathymetry depth (wet/dry vertex depths)
     const unsigned char* wet_in;
@@ -191,7 +259,6 @@ struct StageArgs {
     int stage_index, nstages;  // this stage and the stages per step (the NaN report's stage counter)
     int ne;
     int ne_pad;
-    int n_edges;  // total edge records (stride of egeo)
     double g;
     double h_o, h_o_thr;
     int fn_set;
@@ -203,7 +270,8 @@ struct StageArgs {
     double friction_cf;
     const Real* manning;  // [ne_pad] g n^2 per element (Manning)
     const double* fval;   // [n_forced][NG] this stage's tide / flow values at the forced faces' Gauss points
-    // levee interface fluxes of this stage, [n_levee][2][3][NG] (levee.cu): in side, then ex side
+    // levee interface fluxes of this stage, [n_levee][2][3][NG] (levee.cu): in side, then ex side; zero where both
+    // sides are dry
     const double* levF;
     unsigned char* went_dry;  // [ne] wet_dry_state.went_completely_dry of the last wet/dry pass, or null
     int reverse;              // visit the tiles in reverse order (grid = one CTA per tile)
@@ -258,29 +326,44 @@ __device__ __forceinline__ void llf_flux(Real gravity, const Real qin[3], const 
     F[2] = Real(0.5) * (f2 + e2 + lam * (qin[2] - qex[2]));
 }
 
-// the same flux in packed FP32 (FFMA2 / FMUL2 / FADD2): the in side in lane x, the ex side in lane y, each
-// lane the scalar formula above with its terms in the same order (sp on the in lane only)
-__device__ __forceinline__ void llf_flux_packed(float gravity, const float qin[3], const float qex[3], float bath,
-                                                float sp, float nx, float ny, float F[3]) {
-    const float2 q0 = make_float2(qin[0], qex[0]), q1 = make_float2(qin[1], qex[1]), q2 = make_float2(qin[2], qex[2]);
-    const float2 N = make_float2(nx, nx), M = make_float2(ny, ny), B = make_float2(bath, bath);
-    const float2 h = __fadd2_rn(q0, B);
-    const float2 ih = make_float2(1.0f / h.x, 1.0f / h.y);
-    const float2 u = __fmul2_rn(q1, ih), v = __fmul2_rn(q2, ih);
-    const float2 un = __ffma2_rn(v, M, __fmul2_rn(u, N));
-    const float spc = (nx * sp) * (nx * sp) + ny * ny;
-    const float2 gh = __fmul2_rn(make_float2(gravity, gravity), h);
-    const float lam = fmaxf(fabsf(un.x) + sqrtf(gh.x * spc), fabsf(un.y) + sqrtf(gh.y * spc));
-    const float2 pe = __fmul2_rn(make_float2(gravity, gravity),
-                                 __ffma2_rn(q0, B, __fmul2_rn(__fmul2_rn(q0, q0), make_float2(0.5f, 0.5f))));
-    const float2 uuh = __fmul2_rn(u, q1), vvh = __fmul2_rn(v, q2), uvh = __fmul2_rn(u, q2);
-    const float2 spv = make_float2(sp, 1.0f);
-    const float2 f0 = __ffma2_rn(q2, M, __fmul2_rn(__fmul2_rn(spv, q1), N));
-    const float2 f1 = __ffma2_rn(uvh, M, __fmul2_rn(__fmul2_rn(spv, __fadd2_rn(uuh, pe)), N));
-    const float2 f2 = __ffma2_rn(__fadd2_rn(vvh, pe), M, __fmul2_rn(__fmul2_rn(spv, uvh), N));
-    F[0] = 0.5f * (f0.x + f0.y + lam * (qin[0] - qex[0]));
-    F[1] = 0.5f * (f1.x + f1.y + lam * (qin[1] - qex[1]));
-    F[2] = 0.5f * (f2.x + f2.y + lam * (qin[2] - qex[2]));
+// One side of a face at a Gauss point: the trace, 1 / h and the wave speed sqrt(g h)
+template <typename Real>
+struct Side {
+    Two<Real> q;  // qx, qy
+    Real ze, b, ih, c;
+};
+template <typename Real>
+__device__ __forceinline__ void complete(Side<Real>& s, Real g) {
+    const Real h = s.ze + s.b;
+    s.ih = Real(1) / h;
+    s.c = sqrt(g * h);
+}
+
+// The LLF flux above (sp = 1) of the own side towards the neighbour n, doubled and times w, along the own
+// outward normal times w, N = w nrm: with qn = q . N and un = qn / h the normal flux of a side is
+// (qn, q un + pe N), the same terms as above with the products regrouped (a few ulps). Every term changes sign
+// exactly when the sides trade places and the normal turns round.
+template <bool PK, typename Real>
+__device__ __forceinline__ void llf_sides(Real g, const Side<Real>& o, const Side<Real>& n, Two<Real> N, Real w, Real& F0,
+                                          Two<Real>& F12) {
+    const Real fo = fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)), fn = fma_rn(n.q.x, N.x, mul_rn(n.q.y, N.y));
+    const Real uo = mul_rn(fo, o.ih), un = mul_rn(fn, n.ih);
+    const Real po = mul_rn(mul_rn(g, o.ze), fma_rn(Real(0.5), o.ze, o.b));
+    const Real pn = mul_rn(mul_rn(g, n.ze), fma_rn(Real(0.5), n.ze, n.b));
+    const Two<Real> go = fma2<PK, Real>(o.q, uo, mul2<PK, Real>(N, po));
+    const Two<Real> gn = fma2<PK, Real>(n.q, un, mul2<PK, Real>(N, pn));
+    const Real lam = fmax(fma_rn(o.c, w, fabs(uo)), fma_rn(n.c, w, fabs(un)));
+    F0 = fma_rn(lam, add_rn(o.ze, -n.ze), add_rn(fo, fn));
+    F12 = fma2<PK, Real>(add2<PK, Real>(o.q, Two<Real>{-n.q.x, -n.q.y}), lam, add2<PK, Real>(go, gn));
+}
+
+// Outward normal of face f times w = (half its length) / |J|: a face's normal is along the gradient of the
+// opposite vertex' barycentric coordinate, and with that length the rows of J^-1 are the vectors themselves
+template <typename Real>
+__device__ __forceinline__ Two<Real> scaled_normal(int f, Real Ji00, Real Ji01, Real Ji10, Real Ji11) {
+    if (f == 0) return {Ji00 + Ji10, Ji01 + Ji11};
+    if (f == 1) return {-Ji00, -Ji01};
+    return {-Ji10, -Ji11};
 }
 
 // land boundary ghost state (normal momentum mirrored) + LLF, rkdg_swe_bc_land.hpp:68-86
@@ -348,28 +431,6 @@ __device__ __noinline__ Val3<Real> fn_eval_dev(int id, const double* P, const dg
     return Val3<Real>{out[0], out[1], out[2]};
 }
 
-// Ghost states of the boundaries with data, out of line (one call site per Gauss point; inlined, the p = 1
-// FP32 kernels spill 50-70 bytes per thread and the wet/dry bowl step took 10 % longer):
-// BC::Function (kind 2): ic_q(t, x_gp) (rkdg_swe_bc_function.hpp:33-50);
-// BC::Tide (kind 3) and BC::Flow (kind 4) (rkdg_swe_bc_tide.hpp:73-100, rkdg_swe_bc_flow.hpp:72-102) from the
-// stage's forcing value (form_step_time): a tide sets the ghost surface elevation to it and keeps the
-// interior momentum; a flow keeps the interior elevation and sets the ghost momentum to it times the
-// outward normal. fi is the face's forcing record.
-template <typename Real>
-__device__ __noinline__ Val3<Real> boundary_ghost(const StageArgs<Real>* Ap, const dgsw_fn_time* T, int kind, int fi,
-                                                  int gp, int ng, Real x, Real y, Real qi0, Real qi1, Real qi2,
-                                                  Real nx, Real ny) {
-    const StageArgs<Real>& A = *Ap;
-    if (kind == 2) {
-        Real qe[3];
-        dgsw_fn_eval<Real>(A.fn_set, A.fn_params, *T, 0, x, y, qe);
-        return Val3<Real>{qe[0], qe[1], qe[2]};
-    }
-    const Real f = (Real)A.fval[fi * ng + gp];
-    if (kind == 4) return Val3<Real>{qi0, f * nx, f * ny};
-    return Val3<Real>{f, qi1, qi2};
-}
-
 // the Manning friction factor g n^2 / h^(1/3), bounded below by the Chezy coefficient (swe_source.hpp:37-42);
 // h^(-1/3) through the reciprocal cube root (the reference's pow(h, 1/3) differs from cbrt by the
 // rounding of 1/3, a few ulps)
@@ -380,32 +441,21 @@ __device__ __forceinline__ Real manning_cf(Real gn2, Real h, Real cf0) {
     return cf;
 }
 
-// The manufactured sine set's source terms inline, with its constants hoisted out of the quadrature
-// loops (the same formulas as dgsw_fn_eval, function_sets.h); every other set goes through fn_eval_dev.
+// The manufactured sine set's source terms inline, with its constants of the stage (sine_constants); every
+// other set goes through fn_eval_dev.
 template <typename Real>
 struct SineSrc {
-    // ze = c1 P, qx = -c2 Q, qy = c2 R, zex = c3 Q, zey = -c3 R, zet = -c4 P, qxx = qyy = c5 P,
-    // qxy = qyx = c5 S, qxt = -c6 Q, qyt = c6 R with P = sx cy, Q = cx cy, R = sx sy, S = cx sy
-    Real k, c1, c2, c3, c5, c6, c0, g, H;  // c0 = 2 c5 - c4 (the continuity source)
-    Real kpi;                              // k / pi = 2 / L
+    Real k, c1, c2, c3, c5, c6, c0, g, H, kpi;
 };
 
 template <typename Real>
-__device__ __forceinline__ SineSrc<Real> sine_src_prepare(const double* P, const dgsw_fn_time& T) {
-    const double k = 2.0 * M_PI / P[0], A = P[1], w = T.s[2], B = P[1] * T.s[2] / (2.0 * k);
-    const double st = T.s[0], ct = T.s[1];
-    SineSrc<Real> S;
-    S.k = (Real)k;
-    S.kpi = (Real)(2.0 / P[0]);
-    S.c1 = (Real)(A * ct);
-    S.c2 = (Real)(B * st);
-    S.c3 = (Real)(A * k * ct);
-    S.c5 = (Real)(B * k * st);
-    S.c6 = (Real)(B * w * ct);
-    S.c0 = (Real)(2.0 * B * k * st - A * w * st);
-    S.g = (Real)P[4];
-    S.H = (Real)P[2];
-    return S;
+__device__ __forceinline__ SineSrc<Real> sine_src_load(const StageTime& T) {
+    const Real* c;
+    if constexpr (sizeof(Real) == 8)
+        c = T.sine;
+    else
+        c = T.sine_f;
+    return SineSrc<Real>{c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9]};
 }
 
 // sin and cos of k x: FP64 through sincospi(2 x / L), whose argument reduction is an exact rounding to an
@@ -431,41 +481,41 @@ __device__ __forceinline__ void rotate_small(double s0, double c0, double e, dou
     c = c0 * ce - s0 * se;
 }
 
-// the set's source at a point from sin / cos of k x and k y
-template <typename Real>
-__device__ __forceinline__ void sine_src_terms(const SineSrc<Real>& S, Real sx, Real cx, Real sy, Real cy,
-                                               Real (&out)[3]) {
-    const Real Pp = sx * cy, Q = cx * cy, R = sx * sy, Sq = cx * sy;
-    const Real qx = -S.c2 * Q, qy = S.c2 * R;
-    const Real zex = S.c3 * Q, zey = -S.c3 * R;
-    const Real qxx = S.c5 * Pp, qxy = S.c5 * Sq;  // qyy = qxx, qyx = qxy
+// the set's source at a point from sin / cos of k x and k y: the terms of fn_sine_source regrouped,
+// S_x = qx_t + (3 qx qxx + qxy qy) / h - qx (qx zex + qy zey) / h^2 + g h zex (qyy = qxx), S_y likewise
+template <bool PK, typename Real>
+__device__ __forceinline__ void sine_src_terms(const SineSrc<Real>& S, Real sx, Real cx, Real sy, Real cy, Real& s0,
+                                               Two<Real>& s12) {
+    const Real Pp = sx * cy, Sq = cx * sy;
+    const Two<Real> QR = {cx * cy, sx * sy};
+    const Two<Real> q = mul2<PK, Real>(QR, Two<Real>{-S.c2, S.c2});    // qx, qy
+    const Two<Real> zd = mul2<PK, Real>(QR, Two<Real>{S.c3, -S.c3});   // zex, zey
+    const Real qxx3 = (Real(3) * S.c5) * Pp, qxy = S.c5 * Sq;
     const Real h = S.c1 * Pp + S.H;
     const Real ih = Real(1) / h;
-    const Real ih2 = ih * ih;
-    out[0] = S.c0 * Pp;
-    out[1] = -S.c6 * Q + (Real(2) * qx * qxx * ih - qx * qx * zex * ih2) +
-             ((qxy * qy + qx * qxx) * ih - qx * qy * zey * ih2) + S.g * h * zex;
-    out[2] = S.c6 * R + ((qxx * qy + qx * qxy) * ih - qx * qy * zex * ih2) + (Real(2) * qy * qxx * ih - qy * qy * zey * ih2) +
-             S.g * h * zey;
+    const Real D = (q.x * zd.x + q.y * zd.y) * ih;
+    const Two<Real> t = fma2<PK, Real>(q, qxx3, mul2<PK, Real>(Two<Real>{q.y, q.x}, qxy));
+    const Two<Real> a = fma2<PK, Real>(zd, S.g * h, mul2<PK, Real>(QR, Two<Real>{-S.c6, S.c6}));
+    s0 = S.c0 * Pp;
+    s12 = fma2<PK, Real>(fma2<PK, Real>(q, -D, t), ih, a);
 }
 
-template <typename Real>
-__device__ __forceinline__ void sine_src_eval(const SineSrc<Real>& S, Real x, Real y, Real (&out)[3]) {
+template <bool PK, typename Real>
+__device__ __forceinline__ void sine_src_eval(const SineSrc<Real>& S, Real x, Real y, Real& s0, Two<Real>& s12) {
     Real sx, cx, sy, cy;
     sine_src_sincos<Real>(S, x, sx, cx);
     sine_src_sincos<Real>(S, y, sy, cy);
-    sine_src_terms<Real>(S, sx, cx, sy, cy, out);
+    sine_src_terms<PK, Real>(S, sx, cx, sy, cy, s0, s12);
 }
 
-// the sine set's source at one point, out of line; its constants are rebuilt from the set's parameters
-// (kernel parameter space) and the stage's time factors (shared memory), so no pointer to a local
-// value is taken
+// the sine set's source at one point, out of line
 template <typename Real>
-__device__ __noinline__ Val3<Real> sine_src_far(const double* params, const dgsw_fn_time* T, Real x, Real y) {
-    const SineSrc<Real> S = sine_src_prepare<Real>(params, *T);
-    Real out[3];
-    sine_src_eval<Real>(S, x, y, out);
-    return Val3<Real>{out[0], out[1], out[2]};
+__device__ __noinline__ Val3<Real> sine_src_far(const StageTime* T, Real x, Real y) {
+    const SineSrc<Real> S = sine_src_load<Real>(*T);
+    Real s0;
+    Two<Real> s12;
+    sine_src_eval<false, Real>(S, x, y, s0, s12);
+    return Val3<Real>{s0, s12.x, s12.y};
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -598,32 +648,11 @@ __device__ __forceinline__ bool wetting_drying(Real (&qv)[3][ND], const double b
 template <int P>
 using MT = ct::Master<P>;
 
-// trace of an element's face F at the edge Gauss points: ze, qx, qy and bathymetry,
-// sum over the modes in ascending order (same arithmetic for tile and halo elements)
-template <int P, int F, typename Real, bool PK = false>
+// trace of an element's face F at the edge Gauss points: ze, qx, qy and bathymetry (the levee and trouble passes)
+template <int P, int F, typename Real>
 __device__ __forceinline__ void face_trace(const Real (&q)[3][MT<P>::ND], const Real (&b)[3],
                                            Real (&t)[4][MT<P>::NG]) {
     constexpr int ND = MT<P>::ND, NG = MT<P>::NG;
-    if constexpr (PK) {
-        // packed FP32: (ze, qx) and (qy, bathymetry) share each mode's coefficient
-        sfor<0, NG>([&](auto G) {
-            constexpr int g = decltype(G)::value;
-            Real s0 = Real(0), s1 = Real(0), s2 = Real(0), sb = Real(0);
-            sfor<0, ND>([&](auto K) {
-                constexpr int k = decltype(K)::value;
-                constexpr double c = MT<P>::fphi((F * ND + k) * NG + g);
-                if constexpr (c != 0.0) {
-                    fma_pair(s0, s1, q[0][k], q[1][k], (Real)c, (Real)c);
-                    if constexpr (k < 3)
-                        fma_pair(s2, sb, q[2][k], b[k], (Real)c, (Real)c);
-                    else
-                        s2 = __fmaf_rn(q[2][k], (Real)c, s2);
-                }
-            });
-            t[0][g] = s0, t[1][g] = s1, t[2][g] = s2, t[3][g] = sb;
-        });
-        return;
-    }
     sfor<0, NG>([&](auto G) {
         constexpr int g = decltype(G)::value;
         sfor<0, 3>([&](auto V) {
@@ -646,90 +675,285 @@ __device__ __forceinline__ void face_trace(const Real (&q)[3][MT<P>::ND], const 
     });
 }
 
-// the same trace for a face known only at run time, with the face's basis values from a [mode][gp] table:
-// the halo faces of a warp belong to different faces, and one compile-time copy per face would split the
-// warp. Entries that are zero on this face but not on another add a zero product (the sum is unchanged), so
-// the values equal face_trace's bit for bit.
-template <int P, typename Real, bool PK = false>
-__device__ __forceinline__ void face_trace_rt(const Real (&q)[3][MT<P>::ND], const Real (&b)[3], const Real* cf,
-                                              Real (&t)[4][MT<P>::NG]) {
-    constexpr int ND = MT<P>::ND, NG = MT<P>::NG;
-    if constexpr (PK) {
-        sfor<0, NG>([&](auto G) {
-            constexpr int g = decltype(G)::value;
-            Real s0 = Real(0), s1 = Real(0), s2 = Real(0), sb = Real(0);
-            sfor<0, ND>([&](auto K) {
-                constexpr int k = decltype(K)::value;
-                constexpr bool used = MT<P>::fphi((0 * ND + k) * NG + g) != 0.0 ||
-                                      MT<P>::fphi((1 * ND + k) * NG + g) != 0.0 ||
-                                      MT<P>::fphi((2 * ND + k) * NG + g) != 0.0;
-                if constexpr (used) {
-                    const Real c = cf[k * NG + g];
-                    fma_pair(s0, s1, q[0][k], q[1][k], c, c);
-                    if constexpr (k < 3)
-                        fma_pair(s2, sb, q[2][k], b[k], c, c);
-                    else
-                        s2 = __fmaf_rn(q[2][k], c, s2);
-                }
-            });
-            t[0][g] = s0, t[1][g] = s1, t[2][g] = s2, t[3][g] = sb;
-        });
-        return;
+// Trace slots in shared memory, 16-byte vectors [vector][NS slots]: FP32 one vector (qx, qy, ze, b) per Gauss
+// point; FP64 three, (qx, qy), (ze, b) and (1 / h, sqrt(g h)), so that the divisions and square roots are
+// taken once per trace and not by both sides. A thread's slots are three apart: its 16-byte accesses meet
+// the banks without conflicts.
+template <int P, typename Real>
+struct Trace {
+    static constexpr int NG = MT<P>::NG;
+    static constexpr int NV = sizeof(Real) == 8 ? 3 : 1;  // vectors per Gauss point
+    static __device__ __forceinline__ void put(unsigned char* tr, int NS, int slot, int gp, const Side<Real>& s) {
+        if constexpr (sizeof(Real) == 4) {
+            reinterpret_cast<float4*>(tr)[gp * NS + slot] = make_float4(s.q.x, s.q.y, s.ze, s.b);
+        } else {
+            double2* v = reinterpret_cast<double2*>(tr) + gp * NV * NS + slot;
+            v[0] = make_double2(s.q.x, s.q.y);
+            v[NS] = make_double2(s.ze, s.b);
+            v[2 * NS] = make_double2(s.ih, s.c);
+        }
     }
-    sfor<0, NG>([&](auto G) {
-        constexpr int g = decltype(G)::value;
-        sfor<0, 3>([&](auto V) {
-            constexpr int v = decltype(V)::value;
-            Real s = Real(0);
-            sfor<0, ND>([&](auto K) {
-                constexpr int k = decltype(K)::value;
-                constexpr bool used = MT<P>::fphi((0 * ND + k) * NG + g) != 0.0 ||
-                                      MT<P>::fphi((1 * ND + k) * NG + g) != 0.0 ||
-                                      MT<P>::fphi((2 * ND + k) * NG + g) != 0.0;
-                if constexpr (used) s += q[v][k] * cf[k * NG + g];
-            });
-            t[v][g] = s;
-        });
-        Real sb = Real(0);
-        sfor<0, 3>([&](auto K) {
-            constexpr int k = decltype(K)::value;
-            constexpr bool used = MT<P>::fphi((0 * ND + k) * NG + g) != 0.0 ||
-                                  MT<P>::fphi((1 * ND + k) * NG + g) != 0.0 ||
-                                  MT<P>::fphi((2 * ND + k) * NG + g) != 0.0;
-            if constexpr (used) sb += b[k] * cf[k * NG + g];
-        });
-        t[3][g] = sb;
+    static __device__ __forceinline__ Side<Real> get(const unsigned char* tr, int NS, int slot, int gp, Real g) {
+        Side<Real> s;
+        if constexpr (sizeof(Real) == 4) {
+            const float4 v = reinterpret_cast<const float4*>(tr)[gp * NS + slot];
+            s.q = {v.x, v.y}, s.ze = v.z, s.b = v.w;
+            complete<Real>(s, g);
+        } else {
+            const double2* v = reinterpret_cast<const double2*>(tr) + gp * NV * NS + slot;
+            const double2 a = v[0], b = v[NS], c = v[2 * NS];
+            s.q = {a.x, a.y}, s.ze = b.x, s.b = b.y, s.ih = c.x, s.c = c.y;
+        }
+        return s;
+    }
+};
+
+// the trace of an element's face F at Gauss point G: sums over the modes in ascending order (the same
+// arithmetic for tile and halo elements)
+template <int P, int F, int G, bool PK, typename Real>
+__device__ __forceinline__ Side<Real> face_point(const Real (&q)[3][MT<P>::ND], const Real (&b)[3]) {
+    constexpr int ND = MT<P>::ND, NG = MT<P>::NG;
+    Two<Real> s12 = {Real(0), Real(0)}, s0b = {Real(0), Real(0)};
+    sfor<0, ND>([&](auto K) {
+        constexpr int k = decltype(K)::value;
+        constexpr double c = MT<P>::fphi((F * ND + k) * NG + G);
+        if constexpr (counts(c)) {
+            s12 = fma2<PK, Real>(Two<Real>{q[1][k], q[2][k]}, (Real)c, s12);
+            if constexpr (k < 3)
+                s0b = fma2<PK, Real>(Two<Real>{q[0][k], b[k]}, (Real)c, s0b);
+            else
+                s0b.x = fma_rn(q[0][k], (Real)c, s0b.x);
+        }
+    });
+    Side<Real> s;
+    s.q = s12, s.ze = s0b.x, s.b = s0b.y, s.ih = s.c = Real(0);
+    return s;
+}
+// `whole` false: a dry element's face in a wet/dry kernel, whose 1 / h and sqrt(g h) only the interfaces with one
+// dry side would read; they form it themselves
+template <int P, int F, bool PK, typename Real>
+__device__ __forceinline__ void put_face(unsigned char* tr, int NS, int slot, const Real (&q)[3][MT<P>::ND],
+                                         const Real (&b)[3], Real g, bool whole) {
+    sfor<0, MT<P>::NG>([&](auto G) {
+        constexpr int gp = decltype(G)::value;
+        Side<Real> s = face_point<P, F, gp, PK, Real>(q, b);
+        if (sizeof(Real) == 8 && whole) complete<Real>(s, g);
+        Trace<P, Real>::put(tr, NS, slot, gp, s);
     });
 }
 
-// shared-memory layout of the stage kernel
-template <int P, typename Real, bool WD>
+// the same for a face known only at run time, with the face's basis values from a [mode][gp] table: the halo
+// faces of a warp belong to different faces, and one compile-time copy per face would split the warp.
+// Entries that are zero on this face but not on another add a zero product (the sum is unchanged), so the
+// values equal put_face's bit for bit.
+template <int P, bool PK, typename Real>
+__device__ __forceinline__ void put_face_rt(unsigned char* tr, int NS, int slot, const Real (&q)[3][MT<P>::ND],
+                                            const Real (&b)[3], const Real* cf, Real g) {
+    constexpr int ND = MT<P>::ND, NG = MT<P>::NG;
+    sfor<0, NG>([&](auto G) {
+        constexpr int gp = decltype(G)::value;
+        Two<Real> s12 = {Real(0), Real(0)}, s0b = {Real(0), Real(0)};
+        sfor<0, ND>([&](auto K) {
+            constexpr int k = decltype(K)::value;
+            constexpr bool used = counts(MT<P>::fphi((0 * ND + k) * NG + gp)) ||
+                                  counts(MT<P>::fphi((1 * ND + k) * NG + gp)) ||
+                                  counts(MT<P>::fphi((2 * ND + k) * NG + gp));
+            if constexpr (used) {
+                const Real c = cf[k * NG + gp];
+                s12 = fma2<PK, Real>(Two<Real>{q[1][k], q[2][k]}, c, s12);
+                if constexpr (k < 3)
+                    s0b = fma2<PK, Real>(Two<Real>{q[0][k], b[k]}, c, s0b);
+                else
+                    s0b.x = fma_rn(q[0][k], c, s0b.x);
+            }
+        });
+        Side<Real> s;
+        s.q = s12, s.ze = s0b.x, s.b = s0b.y;
+        if constexpr (sizeof(Real) == 8) complete<Real>(s, g);
+        Trace<P, Real>::put(tr, NS, slot, gp, s);
+    });
+}
+
+// A boundary face's ghost states into its trace slot, at the Gauss points as a neighbour across the face
+// would number them; out of line (boundary elements only). own: the face's own trace slot.
+// BC::Land: normal momentum mirrored (rkdg_swe_bc_land.hpp:44-56); BC::Function: ic_q(t, x_gp)
+// (rkdg_swe_bc_function.hpp:33-50); BC::Tide and BC::Flow (rkdg_swe_bc_tide.hpp:73-100,
+// rkdg_swe_bc_flow.hpp:72-102) from the stage's forcing values (form_step_time): a tide sets the ghost
+// surface elevation and keeps the interior momentum; a flow keeps the interior elevation and sets the ghost
+// momentum to the value times the outward normal. All of them keep the interior bathymetry.
+template <int P, typename Real>
+__device__ __noinline__ void ghost_face(const StageArgs<Real>* Ap, unsigned char* tr, int NS, int own, int slot, int d,
+                                        int f, int kind, int forcing, Real nx, Real ny) {
+    const StageArgs<Real>& A = *Ap;
+    constexpr int NG = MT<P>::NG;
+    const Real g = (Real)A.g;
+    double xa = 0, ya = 0, xb = 0, yb = 0;
+    if (kind == 2) {
+        // the Gauss points lie on the segment from node (f+1)%3 to node (f+2)%3
+        const double2 pa = A.xy[A.enodes[((f + 1) % 3) * A.ne_pad + d]];
+        const double2 pb = A.xy[A.enodes[((f + 2) % 3) * A.ne_pad + d]];
+        xa = pa.x, ya = pa.y, xb = pb.x, yb = pb.y;
+    }
+    sfor<0, NG>([&](auto GP) {
+        constexpr int gp = decltype(GP)::value;
+        constexpr double wa = MT<P>::fpsi((0 * 3 + 1) * NG + gp), wb = MT<P>::fpsi((0 * 3 + 2) * NG + gp);
+        Side<Real> s = Trace<P, Real>::get(tr, NS, own, gp, g);
+        if (kind == 1) {
+            const Real tx = -ny, ty = nx;
+            const Real qn = -(s.q.x * nx + s.q.y * ny);
+            const Real qt = s.q.x * tx + s.q.y * ty;
+            s.q = {qn * nx + qt * tx, qn * ny + qt * ty};
+        } else if (kind == 2) {
+            Real qe[3];
+            dgsw_fn_eval<Real>(A.fn_set, A.fn_params, A.clock->at[A.stage_index].ft, 0, (Real)(xa * wa + xb * wb),
+                               (Real)(ya * wa + yb * wb), qe);
+            s.ze = qe[0], s.q = {qe[1], qe[2]};
+        } else {
+            const Real v = (Real)A.fval[forcing * NG + gp];
+            if (kind == 4)
+                s.q = {v * nx, v * ny};
+            else
+                s.ze = v;
+        }
+        if constexpr (sizeof(Real) == 8) complete<Real>(s, g);
+        Trace<P, Real>::put(tr, NS, slot, NG - 1 - gp, s);
+    });
+}
+
+// the spherical correction at Gauss point gp of face f
+template <int P, typename Real>
+__device__ __forceinline__ Real spherical_factor(const StageArgs<Real>& A, int d, int f, int gp) {
+    constexpr int NG = MT<P>::NG;
+    const double ya = A.xy[A.enodes[((f + 1) % 3) * A.ne_pad + d]].y, yb = A.xy[A.enodes[((f + 2) % 3) * A.ne_pad + d]].y;
+    double wa = 0, wb = 0;
+    sfor<0, NG>([&](auto GP) {
+        constexpr int k = decltype(GP)::value;
+        if (gp == k) wa = MT<P>::fpsi((0 * 3 + 1) * NG + k), wb = MT<P>::fpsi((0 * 3 + 2) * NG + k);
+    });
+    return (Real)(A.sp_cos_lat0 / cos((ya * wa + yb * wb) / A.sp_R));
+}
+
+// The wet/dry fix-ups of an interface (wd_fixup) seen from one of its elements: own and neighbour are put into
+// the interface's in / ex order, and the own side's doubled flux times w comes back (F likewise). Out of line (interfaces with a
+// dry side only).
+template <int P, typename Real>
+__device__ __noinline__ Val3<Real> wd_fixup_own(const StageArgs<Real>* Ap, int d, int f, int gp, bool is_in, bool wo,
+                                                bool wn, Real oz, Real ox, Real oy, Real ob, Real nz, Real nqx, Real nqy,
+                                                Real nb, Real Nx, Real Ny, Real w, Real F0, Real F1, Real F2) {
+    const StageArgs<Real>& A = *Ap;
+    Real sp = Real(1);
+    if (A.spherical) sp = spherical_factor<P, Real>(A, d, f, gp);
+    const Real g = (Real)A.g, half = Real(0.5) / w, nx = Nx / w, ny = Ny / w, w2 = 2 * w;
+    if (is_in) {
+        const Flux2<Real> r = wd_fixup<Real>(g, oz, ox, oy, nz, nqx, nqy, ob, nb, sp, nx, ny, wo, wn, half * F0, half * F1,
+                                             half * F2);
+        return Val3<Real>{w2 * r.i0, w2 * r.i1, w2 * r.i2};
+    }
+    const Flux2<Real> r = wd_fixup<Real>(g, nz, nqx, nqy, oz, ox, oy, nb, ob, sp, -nx, -ny, wn, wo, -half * F0, -half * F1,
+                                         -half * F2);
+    return Val3<Real>{w2 * r.e0, w2 * r.e1, w2 * r.e2};
+}
+
+// the doubled flux times w of an own side towards n where the spherical correction (sp on the interface's in side
+// only) applies; out of line
+template <int P, typename Real>
+__device__ __noinline__ Val3<Real> spherical_flux(const StageArgs<Real>* Ap, int d, int f, int gp, bool is_in, Real oz,
+                                                  Real ox, Real oy, Real ob, Real nz, Real nqx, Real nqy, Real nb,
+                                                  Real Nx, Real Ny, Real w) {
+    const StageArgs<Real>& A = *Ap;
+    const Real sp = spherical_factor<P, Real>(A, d, f, gp);
+    const Real qo[3] = {oz, ox, oy}, qn[3] = {nz, nqx, nqy};
+    const Real nx = Nx / w, ny = Ny / w, w2 = 2 * w;
+    Real F[3];
+    if (is_in) {
+        llf_flux<Real>((Real)A.g, qo, qn, ob, sp, nx, ny, F);
+        return Val3<Real>{F[0] * w2, F[1] * w2, F[2] * w2};
+    }
+    llf_flux<Real>((Real)A.g, qn, qo, nb, sp, -nx, -ny, F);
+    return Val3<Real>{-F[0] * w2, -F[1] * w2, -F[2] * w2};
+}
+
+// The master tables in constant memory, for the loops that run rolled (uniform indexes); FP32 entries twice,
+// as the operand of a packed instruction
+template <typename Real>
+struct CoefType {
+    using type = Real;
+};
+template <>
+struct CoefType<float> {
+    using type = Two<float>;
+};
+template <typename Real>
+using Coef = typename CoefType<Real>::type;
+__host__ __device__ constexpr Two<float> as_coef(float c) { return {c, c}; }
+__host__ __device__ constexpr double as_coef(double c) { return c; }
+__device__ __forceinline__ Two<float> pair_of(Two<float> c) { return c; }
+__device__ __forceinline__ Two<double> pair_of(double c) { return {c, c}; }
+
+template <int P, typename Real>
+struct StageTab {
+    static constexpr int ND = MT<P>::ND, NQ = MT<P>::NQ, NG = MT<P>::NG;
+    Coef<Real> phi[NQ][ND], m0[NQ][ND], m1[NQ][ND], pw[NQ][ND];
+    Real psi[NQ][4];
+    Coef<Real> fphi[3][NG][ND];
+    Real gw[NG];
+};
+template <int P, typename Real>
+constexpr StageTab<P, Real> make_stage_tab() {
+    using T = StageTab<P, Real>;
+    T t{};
+    for (int q = 0; q < T::NQ; ++q) {
+        for (int k = 0; k < T::ND; ++k) {
+            t.phi[q][k] = as_coef((Real)MT<P>::phi(k * T::NQ + q));
+            t.m0[q][k] = as_coef((Real)MT<P>::mz((0 * T::NQ + q) * T::ND + k));
+            t.m1[q][k] = as_coef((Real)MT<P>::mz((1 * T::NQ + q) * T::ND + k));
+            t.pw[q][k] = as_coef((Real)MT<P>::phiw(q * T::ND + k));
+        }
+        for (int n = 0; n < 3; ++n) t.psi[q][n] = (Real)MT<P>::psi(n * T::NQ + q);
+    }
+    for (int g = 0; g < T::NG; ++g) t.gw[g] = (Real)MT<P>::gw(g);
+    for (int f = 0; f < 3; ++f)
+        for (int g = 0; g < T::NG; ++g)
+            for (int k = 0; k < T::ND; ++k) t.fphi[f][g][k] = as_coef((Real)MT<P>::fphi((f * T::ND + k) * T::NG + g));
+    return t;
+}
+template <int P, typename Real>
+__constant__ const StageTab<P, Real> stage_tab = make_stage_tab<P, Real>();
+
+// whether mode k's entry counts at any point (0: phi, 1: m0, 2: m1, 3: pw, 4: fphi)
+template <int P>
+constexpr bool counts_any(int what, int k) {
+    using M = MT<P>;
+    if (what == 4) {
+        for (int i = 0; i < 3 * M::NG; ++i)
+            if (counts(M::fphi((i / M::NG * M::ND + k) * M::NG + i % M::NG))) return true;
+        return false;
+    }
+    for (int q = 0; q < M::NQ; ++q)
+        if (counts(what == 0   ? M::phi(k * M::NQ + q)
+                   : what == 1 ? M::mz((0 * M::NQ + q) * M::ND + k)
+                   : what == 2 ? M::mz((1 * M::NQ + q) * M::ND + k)
+                               : M::phiw(q * M::ND + k)))
+            return true;
+    return false;
+}
+
+// shared-memory layout of the stage kernel; mh: halo and boundary faces of a tile
+template <int P, typename Real>
 struct Smem {
-    static constexpr int ND = MT<P>::ND, NG = MT<P>::NG;
-    static constexpr int NTC = 4 * NG;                 // trace components per face slot
-    static constexpr int NFC = (WD ? 2 : 1) * 3 * NG;  // flux components stored per edge
+    static constexpr int ND = MT<P>::ND;
     static __host__ __device__ size_t al(size_t b) { return (b + 15) & ~size_t(15); }
     static __host__ __device__ int nslot(int tile, int mh) { return 3 * tile + mh; }
-    static __host__ __device__ size_t off_tr(int) { return 0; }
-    static __host__ __device__ size_t off_F(int tile, int mh) {
-        return off_tr(tile) + al(sizeof(Real) * (size_t)NTC * nslot(tile, mh));
-    }
-    static __host__ __device__ size_t off_sJ(int tile, int mh, int me) {
-        return off_F(tile, mh) + al(sizeof(Real) * (size_t)NFC * me);
-    }
-    static __host__ __device__ size_t off_wet(int tile, int mh, int me) {
-        return off_sJ(tile, mh, me) + al(sizeof(Real) * (size_t)me);
-    }
-    static __host__ __device__ size_t off_flag(int tile, int mh, int me) {
-        return off_wet(tile, mh, me) + al((size_t)nslot(tile, mh));
+    static __host__ __device__ size_t off_wet(int tile, int mh) {
+        return (size_t)16 * MT<P>::NG * Trace<P, Real>::NV * nslot(tile, mh);
     }
     // halo staging: the state and bathymetry modes of each halo face's element, copied asynchronously
-    static __host__ __device__ size_t off_halo(int tile, int mh, int me) { return off_flag(tile, mh, me) + al((size_t)me); }
-    static __host__ __device__ size_t off_hbath(int tile, int mh, int me) {
-        return off_halo(tile, mh, me) + al(sizeof(double) * (size_t)3 * ND * mh);
+    static __host__ __device__ size_t off_halo(int tile, int mh) { return off_wet(tile, mh) + al((size_t)nslot(tile, mh)); }
+    static __host__ __device__ size_t off_hbath(int tile, int mh) {
+        return off_halo(tile, mh) + al(sizeof(double) * (size_t)3 * ND * mh);
     }
-    static __host__ __device__ size_t bytes(int tile, int mh, int me) {
-        return off_hbath(tile, mh, me) + al(sizeof(Real) * (size_t)3 * mh);
+    static __host__ __device__ size_t bytes(int tile, int mh) {
+        return off_hbath(tile, mh) + al(sizeof(Real) * (size_t)3 * mh);
     }
 };
 
@@ -750,8 +974,9 @@ __device__ __forceinline__ void cp_async_commit_and_wait() {
 // resident CTAs per SM the register budget is sized for (p = 1 and p = 2 separately; measured at tile
 // 128 on 524,288 triangles: p = 2 FP32 4 (5 spills 592 B and runs 40 % slower), p = 1 FP32 5 (3-9 %
 // faster than 4 on the bowl, tidal, levee and manufactured workloads; 6 spills and is slower), p = 2
-// FP64 3, p = 1 FP64 4 without wetting/drying (14-15 % faster than 3 on the tidal, levee and
-// manufactured workloads) and 3 with it (4 spills in the wet/dry pass and is 6 % slower on the bowl))
+// FP64 3, p = 1 FP64 4 without wetting/drying or analytic source (the tidal channel 0.96 against 1.07 ms per 8
+// steps), 3 with the source (4 spills: 1.63 against 1.36 ms) and with wetting/drying (bowl of 131,072 0.55 against
+// 0.57 ms; of 980,000 3.10 against 2.86 ms, but 3 for the smaller ones))
 #ifndef DGSW_F32_MB128
 #define DGSW_F32_MB128 4
 #endif
@@ -764,66 +989,72 @@ __device__ __forceinline__ void cp_async_commit_and_wait() {
 #ifndef DGSW_F64_P1_MB128
 #define DGSW_F64_P1_MB128 4
 #endif
+#ifndef DGSW_F64_P1_FSRC_MB128
+#define DGSW_F64_P1_FSRC_MB128 3
+#endif
 #ifndef DGSW_F64_P1_WD_MB128
 #define DGSW_F64_P1_WD_MB128 3
 #endif
 // OCC = 1 selects the autotuner's alternative budget: one resident CTA fewer where the default holds
 // several (more registers per thread), one more where it holds one (tile 256 in FP64)
-template <int P, typename Real, int TILE, bool WD, int OCC = 0>
+template <int P, typename Real, int TILE, bool WD, bool FSRC, int OCC = 0>
 struct MinBlocks {
     static constexpr int f32 = P == 1 ? DGSW_F32_P1_MB128 : DGSW_F32_MB128;
-    static constexpr int f64 = P == 1 ? (WD ? DGSW_F64_P1_WD_MB128 : DGSW_F64_P1_MB128) : DGSW_F64_MB128;
+    static constexpr int f64 = P == 1 ? (WD ? DGSW_F64_P1_WD_MB128 : FSRC ? DGSW_F64_P1_FSRC_MB128 : DGSW_F64_P1_MB128)
+                                      : DGSW_F64_MB128;
     static constexpr int base = sizeof(Real) == 4 ? (TILE == 128 ? f32 : 2) : (TILE == 128 ? f64 : 1);
     static constexpr int value = OCC == 0 ? base : (base > 1 ? base - 1 : base + 1);
 };
 
-// shared-memory capacities a tile almost always fits (measured: about 0.27 TILE halo faces and 1.65 TILE
-// edges on structured and jittered meshes); with CAPPED the trace and flux strides are these
-// compile-time constants, so every shared-memory access has an immediate offset
+// shared-memory capacity a tile almost always fits (measured: about 0.27 TILE halo faces on structured and
+// jittered meshes); with CAPPED the stride of the trace vectors is this compile-time constant, so every
+// shared-memory access has an immediate offset
 template <int TILE>
 struct TileCap {
     static constexpr int halo = TILE / 2;
-    static constexpr int edges = TILE + TILE / 2 + TILE / 4 + 16;  // 240 for 128, 464 for 256
 };
 
+// the CTA's one barrier: warps arrive with their traces written and wait after the volume integral
+__device__ __forceinline__ void stage_bar_init(unsigned long long* bar, unsigned warps) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(warps)
+                 : "memory");
+}
+__device__ __forceinline__ void stage_bar_arrive(unsigned long long* bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+        asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(bar))
+                     : "memory");
+}
+__device__ __forceinline__ bool stage_bar_wait(unsigned long long* bar) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
+    for (unsigned i = 0; i < (1u << 24); ++i) {
+        unsigned done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(a)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
 template <int P, typename Real, bool WD, bool FSRC, bool FRIC, int TILE, bool CAPPED, int OCC = 0, bool SPLIT = false>
-__global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::value))
-    rkdg_stage_kernel(const __grid_constant__ StageArgs<Real> A, int max_halo_rt, int max_edges_rt) {
+__global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>::value))
+    rkdg_stage_kernel(const __grid_constant__ StageArgs<Real> A, int max_halo_rt) {
     static_assert(!SPLIT || (!WD && sizeof(Real) == 4), "stage increments: FP32 arithmetic without wetting/drying");
     const int max_halo = CAPPED ? TileCap<TILE>::halo : max_halo_rt;
-    const int max_edges = CAPPED ? TileCap<TILE>::edges : max_edges_rt;
     constexpr int ND = MT<P>::ND, NQ = MT<P>::NQ, NG = MT<P>::NG;
-    using SM = Smem<P, Real, WD>;
-    const int NS = SM::nslot(TILE, max_halo);  // trace slots: 3 per tile element, then halo faces
+    using SM = Smem<P, Real>;
+    using TR = Trace<P, Real>;
+    const int NS = SM::nslot(TILE, max_halo);  // trace slots: 3 per tile element, then halo and boundary faces
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // trace slots: FP32 at p = 2 [NS][NG][ze, qx, qy, b], one 16-byte shared access per Gauss point (a slot is
-    // 36 words, so the 8 threads of a quarter-warp that write consecutive slots hit distinct banks);
-    // otherwise [4*NG][NS]. Measured per step against [4*NG][NS] (same bits): config 2 -1.9 %, tidal p = 2
-    // -1.4 %; at p = 1 (24-word slots, two-way bank conflicts) +1.3 to +1.5 %, so p = 1 keeps the old layout
-    Real* str = reinterpret_cast<Real*>(smem_raw + SM::off_tr(TILE));
-    constexpr bool tr_vec = sizeof(Real) == 4 && P == 2;
-    auto tr_at = [&](int c, int gp, int slot) -> Real& {
-        return tr_vec ? str[(slot * NG + gp) * 4 + c] : str[(c * NG + gp) * NS + slot];
-    };
-    // a face's traces into its slot
-    auto put_trace = [&](int slot, const Real (&t)[4][NG]) {
-        if constexpr (tr_vec) {
-#pragma unroll
-            for (int gg = 0; gg < NG; ++gg)
-                *reinterpret_cast<float4*>(str + (slot * NG + gg) * 4) = make_float4(t[0][gg], t[1][gg], t[2][gg], t[3][gg]);
-        } else {
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int gg = 0; gg < NG; ++gg) str[(c * NG + gg) * NS + slot] = t[c][gg];
-        }
-    };
-    Real* sF = reinterpret_cast<Real*>(smem_raw + SM::off_F(TILE, max_halo));       // [NFC][max_edges]
-    Real* ssJ = reinterpret_cast<Real*>(smem_raw + SM::off_sJ(TILE, max_halo, max_edges));
-    unsigned char* swet = smem_raw + SM::off_wet(TILE, max_halo, max_edges);        // [NS]
-    unsigned char* sflag = smem_raw + SM::off_flag(TILE, max_halo, max_edges);      // [max_edges]
-    double* shq = reinterpret_cast<double*>(smem_raw + SM::off_halo(TILE, max_halo, max_edges));  // [3*ND][max_halo]
-    Real* shb = reinterpret_cast<Real*>(smem_raw + SM::off_hbath(TILE, max_halo, max_edges));      // [3][max_halo]
+    unsigned char* tr = smem_raw;
+    unsigned char* swet = smem_raw + SM::off_wet(TILE, max_halo);                         // [NS]
+    double* shq = reinterpret_cast<double*>(smem_raw + SM::off_halo(TILE, max_halo));     // [3*ND][max_halo]
+    Real* shb = reinterpret_cast<Real*>(smem_raw + SM::off_hbath(TILE, max_halo));        // [3][max_halo]
+    __shared__ unsigned long long bar;
 
     // odd stages walk the tiles backwards: they start on the tiles the previous stage wrote last,
     // whose states are still in L2 (tiles are independent, so the results do not change)
@@ -841,41 +1072,56 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
     const Real g = (Real)A.g;
     const double* __restrict__ qs = A.qk[A.nterms - 1];  // this stage's state
     // the stage's time factors (ESSPRKStepper::GetTimeAtCurrentStage), formed during the previous step
-    const dgsw_fn_time& FT = A.clock->at[A.stage_index].ft;
-    // the face traces' basis values at the edge Gauss points, [face][mode][gp], for phase 3's lift and the
-    // halo traces: the elements of a warp visit their faces in different orders, and compile-time tables per
-    // face split the warp into one branch per face. Measured per step (bit-identical results): FP32 at p = 2
-    // -0.6 to -0.9 %; FP64 at p = 2 -0.6 to +0.5 %, p = 1 +1 to +4 % (the shared-memory loads cost more than
-    // the divergence there), so only FP32 at p = 2 uses it
+    const StageTime& ST = A.clock->at[A.stage_index];
+    const dgsw_fn_time& FT = ST.ft;
+    // the face traces' basis values at the edge Gauss points, [face][mode][gp], for the halo traces. Measured per
+    // step against compile-time tables per face (bit-identical results): FP32 at p = 2 -0.6 to -0.9 %; FP64 at
+    // p = 2 -0.6 to +0.5 %, p = 1 +1 to +4 % (the shared-memory loads cost more than the divergence there), so
+    // only FP32 at p = 2 uses it
     constexpr bool rt_face = P == 2 && sizeof(Real) == 4;
-    // packed FP32 FMAs (fma_pair) in the Gauss-point state evaluation, the face traces, the volume integral and
-    // the lift. Measured per step against the scalar FMAs: config 2 -4.5 %, the tidal channel -3.6 % (p = 2)
-    // and -2 % (p = 1); warp instructions per config-2 stage -8 %. With wetting/drying (p = 1 bowl) the
-    // scalar form stays: packed, the bowl step took 6 % longer.
-    constexpr bool packed = sizeof(Real) == 4 && !WD;
-    __shared__ Real sfphi[3 * ND * NG];
-    if (rt_face && threadIdx.x < 3 * ND * NG) {
+    // packed FP32 instructions (Two) throughout the FP32 kernels
+    constexpr bool PK = sizeof(Real) == 4;
+    __shared__ Real sfphi[rt_face ? 3 * ND * NG : 1];
+    if (tid == 0) stage_bar_init(&bar, TILE / 32);
+    if (rt_face && tid < 3 * ND * NG) {
         Real c = Real(0);
         sfor<0, 3 * ND * NG>([&](auto I) {
             constexpr int i = decltype(I)::value;
-            if (threadIdx.x == i) c = (Real)MT<P>::fphi(i);
+            if (tid == i) c = (Real)MT<P>::fphi(i);
         });
-        sfphi[threadIdx.x] = c;
+        sfphi[tid] = c;
     }
-    if (rt_face) __syncthreads();
+    __syncthreads();
     // the manufactured sine set's source inline, in both precisions; other sets go through fn_eval_dev
     const bool sine_set = FSRC && A.fn_set == DGSW_FN_MANUFACTURED_SINE;
     SineSrc<Real> SS;
-    if (sine_set) SS = sine_src_prepare<Real>(A.fn_params, FT);
+    if (sine_set) SS = sine_src_load<Real>(ST);
 
     Real rhs[3][ND];
 #pragma unroll
     for (int v = 0; v < 3; ++v)
 #pragma unroll
         for (int k = 0; k < ND; ++k) rhs[v][k] = Real(0);
-    // stage increments: the combination's increment terms sum_k a_k d_k + dt b_k sol_k in Real, loaded at
-    // the start of phase 3 (measured: issuing them before the first barrier instead gained nothing on the
-    // p = 2 manufactured and tidal workloads and cost 3 % at p = 1)
+    // rhs += G c with (qx, qy) as one pair
+    auto add_to = [&](int k, Real g0, Two<Real> g12, Two<Real> c) {
+        const Two<Real> r = fma2<PK, Real>(g12, c, Two<Real>{rhs[1][k], rhs[2][k]});
+        rhs[1][k] = r.x, rhs[2][k] = r.y;
+        rhs[0][k] = fma_rn(g0, c.x, rhs[0][k]);
+    };
+    auto both = [](double c) { return Two<Real>{(Real)c, (Real)c}; };
+    const StageTab<P, Real>& TB = stage_tab<P, Real>;
+    // Rolled loops over the quadrature points (ROLL_V) and the faces (ROLL_F), their table entries read from
+    // constant memory; unrolled, every entry is an immediate or a constant operand and zero entries are skipped. The
+    // unrolled p = 2 and FP64 kernels outgrow the instruction caches (3.3 stalls on instruction fetch per issue at
+    // FP64 p = 2). Measured per 8 steps of 524,288 triangles, unrolled -> rolled: FP64 p = 2 5.08 -> 4.53 ms (points)
+    // -> 4.34 ms (points and faces), FP64 p = 1 manufactured 1.41 -> 1.36 ms, the FP64 bowl of 980,000 3.34 -> 3.25 ms;
+    // FP32 p = 2 faces 2.08 -> 2.05 ms, points 2.08 -> 2.22 ms; FP32 p = 1 manufactured, points and faces,
+    // 0.735 -> 0.749 ms; FP64 p = 1 channel 0.96 -> 1.00 ms or more. So the FP32 points and all of FP32 p = 1 stay
+    // unrolled, and FP64 p = 1 without source and wetting/drying.
+    constexpr bool ROLL_V = sizeof(Real) == 8 && (P == 2 || FSRC || WD);
+    constexpr bool ROLL_F = P == 2 || (sizeof(Real) == 8 && (FSRC || WD));
+    // stage increments: the combination's increment terms sum_k a_k d_k + dt b_k sol_k in Real, loaded ahead of
+    // the face loop
     Real dcomb[3][ND];
     auto split_comb = [&]() {
 #pragma unroll
@@ -891,11 +1137,12 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
                 for (int v = 0; v < 3; ++v)
 #pragma unroll
                     for (int k = 0; k < ND; ++k) t[v][k] = dj[(v * ND + k) * P_ + d];
-                if constexpr (packed) {
+                if constexpr (PK) {
 #pragma unroll
                     for (int k = 0; k < ND; ++k) {
-                        fma_pair(dcomb[0][k], dcomb[1][k], t[0][k], t[1][k], aj, aj);
-                        dcomb[2][k] = __fmaf_rn(t[2][k], aj, dcomb[2][k]);
+                        const Two<Real> r = fma2<PK, Real>(Two<Real>{t[1][k], t[2][k]}, aj, Two<Real>{dcomb[1][k], dcomb[2][k]});
+                        dcomb[1][k] = r.x, dcomb[2][k] = r.y;
+                        dcomb[0][k] = fma_rn(t[0][k], aj, dcomb[0][k]);
                     }
                 } else {
 #pragma unroll
@@ -912,11 +1159,12 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
                 for (int v = 0; v < 3; ++v)
 #pragma unroll
                     for (int k = 0; k < ND; ++k) u[v][k] = sj[(v * ND + k) * P_ + d];
-                if constexpr (packed) {
+                if constexpr (PK) {
 #pragma unroll
                     for (int k = 0; k < ND; ++k) {
-                        fma_pair(dcomb[0][k], dcomb[1][k], u[0][k], u[1][k], bj, bj);
-                        dcomb[2][k] = __fmaf_rn(u[2][k], bj, dcomb[2][k]);
+                        const Two<Real> r = fma2<PK, Real>(Two<Real>{u[1][k], u[2][k]}, bj, Two<Real>{dcomb[1][k], dcomb[2][k]});
+                        dcomb[1][k] = r.x, dcomb[2][k] = r.y;
+                        dcomb[0][k] = fma_rn(u[0][k], bj, dcomb[0][k]);
                     }
                 } else {
 #pragma unroll
@@ -927,23 +1175,14 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
             }
         }
     };
-    Real aJ = Real(1);
     bool wet = false;
-    // this element's edge slots for phase 3, loaded now so that the latency is hidden
-    const int2 es = active ? A.eslot[d] : make_int2(0, 0);
-    // with capped tiles (at most TILE / 2 halo faces) thread h < nh owns halo face h: its record is
-    // loaded now and its element's data copied asynchronously into shared memory during phase 1
-    const int hoff = A.tile_halo_off[tile];
-    const int nh = A.tile_halo_off[tile + 1] - hoff;
-    const int eoff = A.tile_edge_off[tile];
-    const int nedge = A.tile_edge_off[tile + 1] - eoff;
-    // FP64: one thread asks L2 for the rows this CTA reads only after phase 1: the RK combination's
-    // earlier stages (phase 3) and the tile's edge records and edge geometry (phase 2), so that those
-    // phases start on L2 hits instead of HBM latency. Bulk prefetches want 16-byte aligned ranges: state
-    // rows start on a multiple of TILE elements, the edge geometry rows are trimmed to whole 16-byte
-    // blocks. Measured on 524,288 triangles: FP64 p = 2 stage 201 -> 199 us (tile 128) and 210 -> 206 us
-    // (tile 256), the config-4 bowl 326 -> 309 us; the FP32 stages were unchanged or up to 2 % slower,
-    // so they do without.
+    // with capped tiles (at most TILE / 2 halo and boundary faces) thread h < nh owns halo face h: its record is
+    // loaded now and its element's data copied asynchronously into shared memory while the own traces are formed
+    const int4 ti = A.tiles[tile];
+    const int hoff = ti.x, nh = ti.y;
+    // FP64: one thread asks L2 for the rows this CTA reads only at its end, the RK combination's earlier
+    // stages, so that those loads start on L2 hits instead of HBM latency. Bulk prefetches want 16-byte aligned
+    // ranges: state rows start on a multiple of TILE elements.
     if (sizeof(Real) == 8 && tid == 0) {
         auto prefetch = [](const void* p, unsigned bytes) {
             if (bytes >= 16)
@@ -954,13 +1193,6 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
             for (int c = 0; c < 3 * ND; ++c) prefetch(A.qk[j] + (size_t)c * P_ + e0, rowb);
             if (A.bdt[j] != 0.0)
                 for (int c = 0; c < 3 * ND; ++c) prefetch(A.solk[j] + (size_t)c * P_ + e0, rowb);
-        }
-        prefetch(A.edges + eoff, (unsigned)nedge * 16u);
-        constexpr int per16 = 16 / (int)sizeof(Real);
-        for (int c = 0; c < 3; ++c) {
-            const int b = c * A.n_edges + eoff, e = b + nedge;
-            const int b16 = (b + per16 - 1) / per16 * per16, e16 = e / per16 * per16;
-            if (e16 > b16) prefetch(A.egeo + b16, (unsigned)(e16 - b16) * (unsigned)sizeof(Real));
         }
     }
     // stage increments, last stage: the carried state's trailing part is read only in the epilogue; one
@@ -1019,446 +1251,291 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
         }
     };
 
-    // ---------------- phase 1: volume + source integrals, face traces ----------------
+    // ---------------- traces ----------------
+    Real q[3][ND], b[3];
+    Real Ji00 = Real(0), Ji01 = Real(0), Ji10 = Real(0), Ji11 = Real(0);
+    double x0 = 0, y0 = 0, x1 = 0, y1 = 0, x2 = 0, y2 = 0;
+    // the vertex coordinates (analytic source, spherical correction). FP64 at p = 2, whose register budget is
+    // tightest, loads them after the traces
+    constexpr bool xy_early = sizeof(Real) == 4 || P == 1;
+    auto load_xy = [&]() {
+        if (FSRC || A.spherical) {
+            const int n0 = A.enodes[d], n1 = A.enodes[P_ + d], n2 = A.enodes[2 * P_ + d];
+            const double2 p0 = A.xy[n0], p1 = A.xy[n1], p2 = A.xy[n2];
+            x0 = p0.x, y0 = p0.y, x1 = p1.x, y1 = p1.y, x2 = p2.x, y2 = p2.y;
+        }
+    };
+    // the faces' weights too, where the register budget holds them across the volume integral
+    constexpr bool fw_early = sizeof(Real) == 4 || P == 1;
+    int meta[3];
+    Real fw[3];
     if (active) {
-        Real q[3][ND], b[3];
         load_state(q, d);
         if (CAPPED && hrec.y >= 0) issue_halo_copies();
 #pragma unroll
         for (int k = 0; k < 3; ++k) b[k] = A.bath[k * P_ + d];
-        const Real Ji00 = A.geo[d], Ji01 = A.geo[P_ + d], Ji10 = A.geo[2 * P_ + d], Ji11 = A.geo[3 * P_ + d];
-        aJ = A.geo[4 * P_ + d];
         wet = A.wet_in[d] != 0;
-        // the vertex coordinates (analytic source, spherical correction), loaded ahead of the wet test so that
-        // the node-index and coordinate loads overlap the state loads instead of following the wet flag.
-        // Measured per step on 524,288 triangles: FP32 p = 2 -1.3 to -1.9 %, p = 1 -3 to -4 % in both
-        // precisions; FP64 p = 2, whose register budget is tightest, +2 to +3 %, so there they follow it.
-        constexpr bool xy_early = sizeof(Real) == 4 || P == 1;
-        double x0 = 0, y0 = 0, x1 = 0, y1 = 0, x2 = 0, y2 = 0;
-        auto load_xy = [&]() {
-            if (FSRC || A.spherical) {
-                const int n0 = A.enodes[d], n1 = A.enodes[P_ + d], n2 = A.enodes[2 * P_ + d];
-                const double2 p0 = A.xy[n0], p1 = A.xy[n1], p2 = A.xy[n2];
-                x0 = p0.x, y0 = p0.y, x1 = p1.x, y1 = p1.y, x2 = p2.x, y2 = p2.y;
-            }
-        };
-        if constexpr (xy_early) load_xy();
-        if (wet) {
-            if constexpr (!xy_early) load_xy();
-            // bathymetry gradient: the projected bathymetry is linear, its gradient constant
-            Real db0 = Real(0), db1 = Real(0);
-            sfor<0, 3>([&](auto K) {
-                constexpr int k = decltype(K)::value;
-                constexpr double c0 = MT<P>::dphi((0 * ND + k) * NQ + 0);
-                constexpr double c1 = MT<P>::dphi((1 * ND + k) * NQ + 0);
-                if constexpr (c0 != 0.0) db0 += b[k] * (Real)c0;
-                if constexpr (c1 != 0.0) db1 += b[k] * (Real)c1;
-            });
-            const Real dbx = db0 * Ji00 + db1 * Ji10;
-            const Real dby = db0 * Ji01 + db1 * Ji11;
-            sfor<0, NQ>([&](auto GP) {
-                constexpr int gp = decltype(GP)::value;
-                Real qg[3];
-                Real bg = Real(0);
-                if constexpr (packed) {
-                    // packed FP32: (ze, qx) and (qy, bathymetry) share each mode's coefficient
-                    qg[0] = qg[1] = qg[2] = Real(0);
-                    sfor<0, ND>([&](auto K) {
-                        constexpr int k = decltype(K)::value;
-                        constexpr double c = MT<P>::phi(k * NQ + gp);
-                        if constexpr (c != 0.0) {
-                            fma_pair(qg[0], qg[1], q[0][k], q[1][k], (Real)c, (Real)c);
-                            if constexpr (k < 3)
-                                fma_pair(qg[2], bg, q[2][k], b[k], (Real)c, (Real)c);
-                            else
-                                qg[2] = __fmaf_rn(q[2][k], (Real)c, qg[2]);
-                        }
-                    });
-                } else {
-                    sfor<0, 3>([&](auto V) {
-                        constexpr int v = decltype(V)::value;
-                        Real s = Real(0);
-                        sfor<0, ND>([&](auto K) {
-                            constexpr int k = decltype(K)::value;
-                            constexpr double c = MT<P>::phi(k * NQ + gp);
-                            if constexpr (c != 0.0) s += q[v][k] * (Real)c;
-                        });
-                        qg[v] = s;
-                    });
-                    sfor<0, 3>([&](auto K) {
-                        constexpr int k = decltype(K)::value;
-                        constexpr double c = MT<P>::phi(k * NQ + gp);
-                        if constexpr (c != 0.0) bg += b[k] * (Real)c;
-                    });
-                }
-                // physical flux, swe_flux.hpp:5-25
-                const Real h = qg[0] + bg;
-                const Real ih = Real(1) / h;
-                const Real u = qg[1] * ih, vv = qg[2] * ih;
-                const Real pe = g * (Real(0.5) * qg[0] * qg[0] + qg[0] * bg);
-                Real Fx[3] = {qg[1], u * qg[1] + pe, u * qg[2]};
-                Real Fy[3] = {qg[2], u * qg[2], vv * qg[2] + pe};
-                double yg = 0.0;
-                if (A.spherical) {
-                    constexpr double s0 = MT<P>::psi(0 * NQ + gp), s1 = MT<P>::psi(1 * NQ + gp),
-                                     s2 = MT<P>::psi(2 * NQ + gp);
-                    yg = y0 * s0 + y1 * s1 + y2 * s2;
-                }
-                if (A.spherical) {
-                    const Real sp = (Real)(A.sp_cos_lat0 / cos(yg / A.sp_R));
 #pragma unroll
-                    for (int v = 0; v < 3; ++v) Fx[v] = sp * Fx[v];
-                }
-                // bathymetry-slope source, swe_source.hpp:15-21 (the analytic source follows in its own loop,
-                // except the manufactured sine set in FP32, added here: its sum then shares the phi w products)
-                Real S[3] = {Real(0), g * (dbx * qg[0]), g * (dby * qg[0])};
-                if constexpr (FSRC && sizeof(Real) == 4) {
-                    if (sine_set) {
-                        constexpr double s0 = MT<P>::psi(0 * NQ + gp), s1 = MT<P>::psi(1 * NQ + gp),
-                                         s2 = MT<P>::psi(2 * NQ + gp);
-                        const Real xg = (Real)x0 * (Real)s0 + (Real)x1 * (Real)s1 + (Real)x2 * (Real)s2;
-                        const Real yg = (Real)y0 * (Real)s0 + (Real)y1 * (Real)s1 + (Real)y2 * (Real)s2;
-                        Real fs[3];
-                        sine_src_eval<Real>(SS, xg, yg, fs);
-                        S[0] = fs[0];
-                        S[1] += fs[1];
-                        S[2] += fs[2];
-                    }
-                }
-                // bottom friction, swe_source.hpp:29-51: S(qx, qy) -= Cf |u| / h (qx, qy), Cf the Chezy
-                // coefficient or, for Manning, max(g n^2 / h^(1/3), Cf); |u| as sqrt(u^2 + v^2) and / h as
-                // * (1 / h) where the reference has hypot and a division (each within an ulp; velocities
-                // are far from hypot's overflow range)
-                if (FRIC) {
-                    const Real cf = A.friction == DGSW_FRICTION_MANNING ? manning_cf<Real>(A.manning[d], h, (Real)A.friction_cf)
-                                                                        : (Real)A.friction_cf;
-                    const Real tau = cf * sqrt(u * u + vv * vv) * ih;
-                    S[1] -= tau * qg[1];
-                    S[2] -= tau * qg[2];
-                }
-                // int F . grad(phi) = sum_gp sum_z (F_x J^-1(z,x) + F_y J^-1(z,y)) dphi_z w
-                if constexpr (packed) {
-                    // packed FP32: ze and qx share each mode's coefficients (qy alone), each mode's terms in the
-                    // scalar loop's order
-                    Real G0[3], G1[3];
+        for (int f = 0; f < 3; ++f) meta[f] = A.fmeta[f * P_ + d];
+        if constexpr (fw_early) {
 #pragma unroll
-                    for (int v = 0; v < 3; ++v) {
-                        G0[v] = Fx[v] * Ji00 + Fy[v] * Ji01;
-                        G1[v] = Fx[v] * Ji10 + Fy[v] * Ji11;
-                    }
-                    sfor<0, ND>([&](auto K) {
-                        constexpr int k = decltype(K)::value;
-                        constexpr double m0 = MT<P>::mz((0 * NQ + gp) * ND + k);
-                        constexpr double m1 = MT<P>::mz((1 * NQ + gp) * ND + k);
-                        constexpr double pw = MT<P>::phiw(gp * ND + k);
-                        if constexpr (m0 != 0.0) {
-                            fma_pair(rhs[0][k], rhs[1][k], G0[0], G0[1], (Real)m0, (Real)m0);
-                            rhs[2][k] = __fmaf_rn(G0[2], (Real)m0, rhs[2][k]);
-                        }
-                        if constexpr (m1 != 0.0) {
-                            fma_pair(rhs[0][k], rhs[1][k], G1[0], G1[1], (Real)m1, (Real)m1);
-                            rhs[2][k] = __fmaf_rn(G1[2], (Real)m1, rhs[2][k]);
-                        }
-                        if constexpr (pw != 0.0) {
-                            fma_pair(rhs[0][k], rhs[1][k], S[0], S[1], (Real)pw, (Real)pw);
-                            rhs[2][k] = __fmaf_rn(S[2], (Real)pw, rhs[2][k]);
-                        }
-                    });
-                    return;
-                }
-                sfor<0, 3>([&](auto V) {
-                    constexpr int v = decltype(V)::value;
-                    const Real G0 = Fx[v] * Ji00 + Fy[v] * Ji01;
-                    const Real G1 = Fx[v] * Ji10 + Fy[v] * Ji11;
-                    sfor<0, ND>([&](auto K) {
-                        constexpr int k = decltype(K)::value;
-                        constexpr double m0 = MT<P>::mz((0 * NQ + gp) * ND + k);
-                        constexpr double m1 = MT<P>::mz((1 * NQ + gp) * ND + k);
-                        constexpr double pw = MT<P>::phiw(gp * ND + k);
-                        Real acc = rhs[v][k];
-                        if constexpr (m0 != 0.0) acc += G0 * (Real)m0;
-                        if constexpr (m1 != 0.0) acc += G1 * (Real)m1;
-                        if constexpr (pw != 0.0) acc += S[v] * (Real)pw;
-                        rhs[v][k] = acc;
-                    });
-                });
-            });
-            // analytic source_q(t, x_gp) (swe_source.hpp:9-14), in a loop of its own so that its
-            // temporaries are not live together with the flux computation's
-            // The manufactured sine set in FP64 on elements small against its wavelength (k times the
-            // largest vertex offset from the centroid <= 0.05): sin and cos once at the centroid, turned to
-            // each quadrature point by rotate_small; the point's offset from the centroid is
-            // sum_i (psi_i - 1/3) (x_i - x_0), its coordinate never formed. Measured on 524,288 triangles at
-            // p = 2: FP64 stage 212 -> 201 us; in FP32 the hardware sine/cosine per point stays cheaper
-            // (114 against 116 us).
-            const double xc = (x0 + x1 + x2) * (1.0 / 3.0), yc = (y0 + y1 + y2) * (1.0 / 3.0);
-            bool near = false;
-            if constexpr (sizeof(Real) == 8)
-                near = sine_set && (double)SS.k * fmax(fmax(fmax(fabs(x0 - xc), fabs(x1 - xc)), fabs(x2 - xc)),
-                                                         fmax(fmax(fabs(y0 - yc), fabs(y1 - yc)), fabs(y2 - yc))) <= 0.05;
-            if constexpr (sizeof(Real) == 8) {
-                if (FSRC && near) {
-                    double sxc, cxc, syc, cyc;
-                    sine_src_sincos<Real>(SS, xc, sxc, cxc);
-                    sine_src_sincos<Real>(SS, yc, syc, cyc);
-                    const double ex1 = x1 - x0, ex2 = x2 - x0, ey1 = y1 - y0, ey2 = y2 - y0;
-                    sfor<0, NQ>([&](auto GP) {
-                        constexpr int gp = decltype(GP)::value;
-                        constexpr double a1 = MT<P>::psi(1 * NQ + gp) - 1.0 / 3.0, a2 = MT<P>::psi(2 * NQ + gp) - 1.0 / 3.0;
-                        double sx, cx, sy, cy;
-                        rotate_small(sxc, cxc, SS.k * (ex1 * a1 + ex2 * a2), sx, cx);
-                        rotate_small(syc, cyc, SS.k * (ey1 * a1 + ey2 * a2), sy, cy);
-                        Real fs[3];
-                        sine_src_terms<Real>(SS, sx, cx, sy, cy, fs);
-                        sfor<0, 3>([&](auto V) {
-                            constexpr int v = decltype(V)::value;
-                            sfor<0, ND>([&](auto K) {
-                                constexpr int k = decltype(K)::value;
-                                constexpr double pw = MT<P>::phiw(gp * ND + k);
-                                if constexpr (pw != 0.0) rhs[v][k] += fs[v] * (Real)pw;
-                            });
-                        });
-                    });
-                }
-            }
-            if (FSRC && !near && !(sizeof(Real) == 4 && sine_set)) {
-                const Real xr0 = (Real)x0, xr1 = (Real)x1, xr2 = (Real)x2;
-                const Real yr0 = (Real)y0, yr1 = (Real)y1, yr2 = (Real)y2;
-                sfor<0, NQ>([&](auto GP) {
-                    constexpr int gp = decltype(GP)::value;
-                    constexpr double s0 = MT<P>::psi(0 * NQ + gp), s1 = MT<P>::psi(1 * NQ + gp),
-                                     s2 = MT<P>::psi(2 * NQ + gp);
-                    // FP32 path: Gauss-point coordinates in FP32 (the analytic source is evaluated in FP32)
-                    const Real xg = xr0 * (Real)s0 + xr1 * (Real)s1 + xr2 * (Real)s2;
-                    const Real yg = yr0 * (Real)s0 + yr1 * (Real)s1 + yr2 * (Real)s2;
-                    Real fs[3];
-                    if (sine_set && sizeof(Real) == 8) {
-                        // FP64 elements large against the wavelength: out of line, so that this rarely
-                        // taken path keeps the kernel's hot code small
-                        const Val3<Real> r = sine_src_far<Real>(A.fn_params, &FT, xg, yg);
-                        fs[0] = r.v0, fs[1] = r.v1, fs[2] = r.v2;
-                    } else if (sine_set) {
-                        sine_src_eval<Real>(SS, xg, yg, fs);
-                    } else {
-                        const Val3<Real> r = fn_eval_dev<Real>(A.fn_set, A.fn_params, &FT, 1, xg, yg);
-                        fs[0] = r.v0, fs[1] = r.v1, fs[2] = r.v2;
-                    }
-                    sfor<0, 3>([&](auto V) {
-                        constexpr int v = decltype(V)::value;
-                        sfor<0, ND>([&](auto K) {
-                            constexpr int k = decltype(K)::value;
-                            constexpr double pw = MT<P>::phiw(gp * ND + k);
-                            if constexpr (pw != 0.0) rhs[v][k] += fs[v] * (Real)pw;
-                        });
-                    });
-                });
-            }
-            // the volume integrals stay in master-element units: sol = (|J| V + E) M^-1 / |J| is
-            // computed as V M^-1 + (E / |J|) M^-1, with 1 / |J| folded into the edge weights below
+            for (int f = 0; f < 3; ++f) fw[f] = A.fw[f * P_ + d];
         }
-        // traces of the three faces (needed also when dry: a wet neighbour evaluates the interface)
+        Ji00 = A.geo[d], Ji01 = A.geo[P_ + d], Ji10 = A.geo[2 * P_ + d], Ji11 = A.geo[3 * P_ + d];
+        if constexpr (xy_early) load_xy();
+        // the three faces (needed also when dry: a wet neighbour evaluates the interface)
         sfor<0, 3>([&](auto FF) {
             constexpr int f = decltype(FF)::value;
-            Real t[4][NG];
-            face_trace<P, f, Real, packed>(q, b, t);
-            const int slot = 3 * tid + f;
-            put_trace(slot, t);
-            swet[slot] = wet ? 1 : 0;
+            put_face<P, f, PK, Real>(tr, NS, 3 * tid + f, q, b, g, !WD || wet);
+            swet[3 * tid + f] = wet ? 1 : 0;
+        });
+        // boundary faces: their ghost states
+        sfor<0, 3>([&](auto FF) {
+            constexpr int f = decltype(FF)::value;
+            const int kind = meta[f] & 7;
+            if (kind >= 1 && kind <= 4) {
+                const int slot = meta[f] >> 4;
+                const Two<Real> N = scaled_normal<Real>(f, Ji00, Ji01, Ji10, Ji11);
+                const Real w = fw_early ? fw[f] : A.fw[f * P_ + d];
+                const int forcing = A.halo[hoff + slot - 3 * TILE].x;
+                ghost_face<P, Real>(&A, tr, NS, 3 * tid + f, slot, d, f, kind, forcing, N.x / w, N.y / w);
+                swet[slot] = wet ? 1 : 0;
+            }
         });
     }
-    // halo faces: faces of elements in other tiles that this tile's edges need
+    // halo faces: faces of elements in other tiles across this tile's edges
+    auto halo_trace = [&](int h, int face, const Real (&qh)[3][ND], const Real (&bh)[3], bool w) {
+        const int slot = 3 * TILE + h;
+        if constexpr (rt_face) {
+            put_face_rt<P, PK, Real>(tr, NS, slot, qh, bh, sfphi + face * ND * NG, g);
+        } else if (face == 0) {
+            put_face<P, 0, PK, Real>(tr, NS, slot, qh, bh, g, !WD || w);
+        } else if (face == 1) {
+            put_face<P, 1, PK, Real>(tr, NS, slot, qh, bh, g, !WD || w);
+        } else {
+            put_face<P, 2, PK, Real>(tr, NS, slot, qh, bh, g, !WD || w);
+        }
+        swet[slot] = w ? 1 : 0;
+    };
     if (CAPPED) {
         if (hrec.y >= 0) {
             if (!active) issue_halo_copies();  // threads past the last element of the last tile
             const int h = tid;
             cp_async_commit_and_wait();  // this thread's own copies
-            Real q[3][ND], b[3], t[4][NG];
+            Real qh[3][ND], bh[3];
             if constexpr (SPLIT) {
                 if (A.dk[A.nterms - 1]) {
 #pragma unroll
                     for (int c = 0; c < 3 * ND; ++c)
-                        q[c / ND][c % ND] = shf[c * max_halo + h] + shf[(3 * ND + c) * max_halo + h];
+                        qh[c / ND][c % ND] = shf[c * max_halo + h] + shf[(3 * ND + c) * max_halo + h];
                 } else {
 #pragma unroll
-                    for (int c = 0; c < 3 * ND; ++c) q[c / ND][c % ND] = shf[c * max_halo + h];
+                    for (int c = 0; c < 3 * ND; ++c) qh[c / ND][c % ND] = shf[c * max_halo + h];
                 }
             } else {
 #pragma unroll
-                for (int c = 0; c < 3 * ND; ++c) q[c / ND][c % ND] = (Real)shq[c * max_halo + h];
+                for (int c = 0; c < 3 * ND; ++c) qh[c / ND][c % ND] = (Real)shq[c * max_halo + h];
             }
 #pragma unroll
-            for (int k = 0; k < 3; ++k) b[k] = shb[k * max_halo + h];
-            if constexpr (rt_face) {
-                face_trace_rt<P, Real, packed>(q, b, sfphi + hrec.y * ND * NG, t);
-            } else if (hrec.y == 0) {
-                face_trace<P, 0, Real, packed>(q, b, t);
-            } else if (hrec.y == 1) {
-                face_trace<P, 1, Real, packed>(q, b, t);
-            } else {
-                face_trace<P, 2, Real, packed>(q, b, t);
-            }
-            const int slot = 3 * TILE + h;
-            put_trace(slot, t);
-            swet[slot] = hwet ? 1 : 0;
+            for (int k = 0; k < 3; ++k) bh[k] = shb[k * max_halo + h];
+            halo_trace(h, hrec.y, qh, bh, hwet);
         }
     } else {
 #pragma unroll 1
         for (int h = tid; h < nh; h += TILE) {
             const int2 it = A.halo[hoff + h];
-            const int e = it.x;
-            Real q[3][ND], b[3], t[4][NG];
-            load_state(q, e);
+            Real qh[3][ND], bh[3];
+            load_state(qh, it.x);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) b[k] = A.bath[k * P_ + e];
-            if constexpr (rt_face) {
-                face_trace_rt<P, Real, packed>(q, b, sfphi + it.y * ND * NG, t);
-            } else if (it.y == 0) {
-                face_trace<P, 0, Real, packed>(q, b, t);
-            } else if (it.y == 1) {
-                face_trace<P, 1, Real, packed>(q, b, t);
-            } else {
-                face_trace<P, 2, Real, packed>(q, b, t);
-            }
-            const int slot = 3 * TILE + h;
-            put_trace(slot, t);
-            swet[slot] = A.wet_in[e] != 0 ? 1 : 0;
+            for (int k = 0; k < 3; ++k) bh[k] = A.bath[k * P_ + it.x];
+            halo_trace(h, it.y, qh, bh, A.wet_in[it.x] != 0);
         }
     }
-    // the first edge record and geometry of phase 2 are loaded before the barrier, so that their latency
-    // overlaps the wait for the CTA's other warps (measured per step on 524,288-2,097,152 triangles: -0.6 to
-    // -1.6 %; FP64 at p = 2, whose register budget is tightest, loads them after the barrier)
-    constexpr bool edge_early = !(sizeof(Real) == 8 && P == 2);
-    int4 rec_e = make_int4(0, 0, 0, 0);
-    Real nx_e = Real(0), ny_e = Real(0), sj_e = Real(0);
-    if (edge_early && tid < nedge) {
-        rec_e = A.edges[eoff + tid];
-        nx_e = A.egeo[eoff + tid];
-        ny_e = A.egeo[A.n_edges + eoff + tid];
-        sj_e = A.egeo[2 * A.n_edges + eoff + tid];
-    }
-    __syncthreads();
+    stage_bar_arrive(&bar);
 
-    // ---------------- phase 2: edge fluxes, once per edge of the tile ----------------
-    {
-        // the next edge's record and geometry are loaded one iteration ahead
-        int4 rec_n = rec_e;
-        Real nx_n = nx_e, ny_n = ny_e, sj_n = sj_e;
-        if (!edge_early && tid < nedge) {
-            rec_n = A.edges[eoff + tid];
-            nx_n = A.egeo[eoff + tid];
-            ny_n = A.egeo[A.n_edges + eoff + tid];
-            sj_n = A.egeo[2 * A.n_edges + eoff + tid];
-        }
-#pragma unroll 1
-        for (int le = tid; le < nedge; le += TILE) {
-            const int4 rec = rec_n;
-            const Real nx = nx_n, ny = ny_n;
-            ssJ[le] = sj_n;
-            if (le + TILE < nedge) {
-                const int nle = eoff + le + TILE;
-                rec_n = A.edges[nle];
-                nx_n = A.egeo[nle];
-                ny_n = A.egeo[A.n_edges + nle];
-                sj_n = A.egeo[2 * A.n_edges + nle];
-            }
-            const int sa = rec.x, sb = rec.y;
-            const int kind = (rec.z >> 4) & 7;
-            const bool wa = swet[sa] != 0;
-            const bool wb = sb >= 0 && swet[sb] != 0;
-            const bool compute = (kind == 0 || kind == 5) ? (wa || wb) : wa;
-            // 2 marks a levee interface: its ex-side flux is not -F and is read in phase 3
-            sflag[le] = compute ? (kind == 5 ? 2 : 1) : 0;
-            if (!compute) continue;
-            if (kind == 5) {
-                // the in-side flux as for any edge; the ex-side flux over the ex face's own trace slot,
-                // which no other edge reads
-                const double* Fl = A.levF + (size_t)(rec.z >> 8) * (6 * NG);
-#pragma unroll
-                for (int c = 0; c < 3 * NG; ++c) sF[c * max_edges + le] = (Real)Fl[c];
-#pragma unroll
-                for (int c = 0; c < 3 * NG; ++c) tr_at(c / NG, c % NG, sb) = (Real)Fl[3 * NG + c];
-                continue;
-            }
-            Real sp = Real(1);
-            double xa = 0, ya = 0, xb = 0, yb = 0;
-            if (kind == 2 || A.spherical) {
-                // Gauss points of face fa lie on the segment from node (fa+1)%3 to node (fa+2)%3
-                const int fa = rec.z & 3, ea = rec.w;
-                const double2 pa = A.xy[A.enodes[((fa + 1) % 3) * P_ + ea]];
-                const double2 pb = A.xy[A.enodes[((fa + 2) % 3) * P_ + ea]];
-                xa = pa.x, ya = pa.y, xb = pb.x, yb = pb.y;
-            }
-            sfor<0, NG>([&](auto GP) {
-                constexpr int gp = decltype(GP)::value;
-                constexpr int ge = NG - 1 - gp;  // the ex side's Gauss point paired with gp
-                // BoundaryToMasterCoordinates + LocalToGlobalCoordinates on a straight edge
-                constexpr double wa_ = MT<P>::fpsi((0 * 3 + 1) * NG + gp), wb_ = MT<P>::fpsi((0 * 3 + 2) * NG + gp);
-                if (A.spherical) sp = (Real)(A.sp_cos_lat0 / cos((ya * wa_ + yb * wb_) / A.sp_R));
-                Real qi[3], bi;
-                if constexpr (tr_vec) {
-                    const float4 a = *reinterpret_cast<const float4*>(str + (sa * NG + gp) * 4);
-                    qi[0] = a.x, qi[1] = a.y, qi[2] = a.z, bi = a.w;
+    // ---------------- volume + source integrals ----------------
+    if (active && wet) {
+        if constexpr (!xy_early) load_xy();
+        // bathymetry gradient: the projected bathymetry is linear, its gradient constant
+        Real db0 = Real(0), db1 = Real(0);
+        sfor<0, 3>([&](auto K) {
+            constexpr int k = decltype(K)::value;
+            constexpr double c0 = MT<P>::dphi((0 * ND + k) * NQ + 0);
+            constexpr double c1 = MT<P>::dphi((1 * ND + k) * NQ + 0);
+            if constexpr (counts(c0)) db0 += b[k] * (Real)c0;
+            if constexpr (counts(c1)) db1 += b[k] * (Real)c1;
+        });
+        const Two<Real> gdb = {g * (db0 * Ji00 + db1 * Ji10), g * (db0 * Ji01 + db1 * Ji11)};
+        auto volume_point = [&](auto GP) {
+            const auto gp = GP;  // IC<gp> (unrolled) or an int
+            Two<Real> m = {Real(0), Real(0)}, zb = {Real(0), Real(0)};  // (qx, qy), (ze, b)
+            sfor<0, ND>([&](auto K) {
+                constexpr int k = decltype(K)::value;
+                auto add = [&](Two<Real> c) {
+                    m = fma2<PK, Real>(Two<Real>{q[1][k], q[2][k]}, c, m);
+                    if constexpr (k < 3)
+                        zb = fma2<PK, Real>(Two<Real>{q[0][k], b[k]}, c, zb);
+                    else
+                        zb.x = fma_rn(q[0][k], c.x, zb.x);
+                };
+                if constexpr (ROLL_V) {
+                    if constexpr (counts_any<P>(0, k)) add(pair_of(TB.phi[gp][k]));
                 } else {
-                    qi[0] = str[(0 * NG + gp) * NS + sa], qi[1] = str[(1 * NG + gp) * NS + sa];
-                    qi[2] = str[(2 * NG + gp) * NS + sa], bi = str[(3 * NG + gp) * NS + sa];
+                    constexpr double c = MT<P>::phi(k * NQ + decltype(GP)::value);
+                    if constexpr (counts(c)) add(both(c));
                 }
-                Real qe[3], be = Real(0);
-                if (kind == 0) {
-                    if constexpr (tr_vec) {
-                        const float4 e = *reinterpret_cast<const float4*>(str + (sb * NG + ge) * 4);
-                        qe[0] = e.x, qe[1] = e.y, qe[2] = e.z;
-                        if (WD) be = e.w;
-                    } else {
-                        qe[0] = str[(0 * NG + ge) * NS + sb];
-                        qe[1] = str[(1 * NG + ge) * NS + sb];
-                        qe[2] = str[(2 * NG + ge) * NS + sb];
-                        if (WD) be = str[(3 * NG + ge) * NS + sb];
-                    }
-                } else if (kind == 1) {
-                    // BC::Land ghost state: normal momentum mirrored (rkdg_swe_bc_land.hpp:44-56)
-                    const Real tx = -ny, ty = nx;
-                    const Real qn_ex = -(qi[1] * nx + qi[2] * ny);
-                    const Real qt_ex = qi[1] * tx + qi[2] * ty;
-                    qe[0] = qi[0];
-                    qe[1] = qn_ex * nx + qt_ex * tx;
-                    qe[2] = qn_ex * ny + qt_ex * ty;
-                } else {
-                    // function, tide and flow boundaries (a tide / flow face's b slot holds -2 - its
-                    // forcing record)
-                    const Val3<Real> r =
-                        boundary_ghost<Real>(&A, &FT, kind, -2 - sb, gp, NG, (Real)(xa * wa_ + xb * wb_),
-                                             (Real)(ya * wa_ + yb * wb_), qi[0], qi[1], qi[2], nx, ny);
-                    qe[0] = r.v0, qe[1] = r.v1, qe[2] = r.v2;
-                }
-                Real Fi[3];
-                // packed at p = 1 only: measured per step, the p = 1 tidal channel -1.7 %; at p = 2 the kernel
-                // spilled and the config-2 step took 2 % longer
-                if constexpr (packed && P == 1)
-                    llf_flux_packed(g, qi, qe, bi, sp, nx, ny, Fi);
-                else
-                    llf_flux<Real>(g, qi, qe, bi, sp, nx, ny, Fi);
-                if (WD && kind == 0) {
-                    Real Fe[3] = {-Fi[0], -Fi[1], -Fi[2]};
-                    if (!(wa && wb)) {
-                        const Flux2<Real> r = wd_fixup<Real>(g, qi[0], qi[1], qi[2], qe[0], qe[1], qe[2], bi, be, sp,
-                                                             nx, ny, wa, wb, Fi[0], Fi[1], Fi[2]);
-                        Fi[0] = r.i0, Fi[1] = r.i1, Fi[2] = r.i2;
-                        Fe[0] = r.e0, Fe[1] = r.e1, Fe[2] = r.e2;
-                    }
-#pragma unroll
-                    for (int v = 0; v < 3; ++v) sF[((3 + v) * NG + gp) * max_edges + le] = Fe[v];
-                }
-#pragma unroll
-                for (int v = 0; v < 3; ++v) sF[(v * NG + gp) * max_edges + le] = Fi[v];
             });
+            // physical flux (swe_flux.hpp:5-25) along the two master directions J^-1(z, :): with the contravariant
+            // momentum U = J^-1(z, 0) qx + J^-1(z, 1) qy it is (U, q U / h + pe J^-1(z, :))
+            const Real h = zb.x + zb.y;
+            const Real ih = Real(1) / h;
+            const Real pe = g * zb.x * (Real(0.5) * zb.x + zb.y);
+            Real X0 = Ji00, X1 = Ji10;
+            if (A.spherical) {
+                const int i = gp;
+                const Real sp = (Real)(A.sp_cos_lat0 / cos((y0 * TB.psi[i][0] + y1 * TB.psi[i][1] + y2 * TB.psi[i][2]) / A.sp_R));
+                X0 *= sp, X1 *= sp;
+            }
+            const Real U0 = X0 * m.x + Ji01 * m.y, U1 = X1 * m.x + Ji11 * m.y;
+            const Two<Real> G0 = fma2<PK, Real>(m, U0 * ih, mul2<PK, Real>(Two<Real>{X0, Ji01}, pe));
+            const Two<Real> G1 = fma2<PK, Real>(m, U1 * ih, mul2<PK, Real>(Two<Real>{X1, Ji11}, pe));
+            // bathymetry-slope source, swe_source.hpp:15-21 (the analytic source follows in its own loop,
+            // except the manufactured sine set in FP32, added here: its sum then shares the phi w products)
+            Real S0 = Real(0);
+            Two<Real> S12 = mul2<PK, Real>(gdb, zb.x);
+            if constexpr (FSRC && sizeof(Real) == 4) {
+                if (sine_set) {
+                    Real s0, s1, s2;
+                    if constexpr (ROLL_V) {
+                        s0 = TB.psi[gp][0], s1 = TB.psi[gp][1], s2 = TB.psi[gp][2];
+                    } else {
+                        constexpr int i = decltype(GP)::value;
+                        s0 = (Real)MT<P>::psi(0 * NQ + i), s1 = (Real)MT<P>::psi(1 * NQ + i), s2 = (Real)MT<P>::psi(2 * NQ + i);
+                    }
+                    const Real xg = (Real)x0 * s0 + (Real)x1 * s1 + (Real)x2 * s2;
+                    const Real yg = (Real)y0 * s0 + (Real)y1 * s1 + (Real)y2 * s2;
+                    Two<Real> fs;
+                    sine_src_eval<PK, Real>(SS, xg, yg, S0, fs);
+                    S12 = add2<PK, Real>(S12, fs);
+                }
+            }
+            // bottom friction, swe_source.hpp:29-51: S(qx, qy) -= Cf |u| / h (qx, qy), Cf the Chezy coefficient
+            // or, for Manning, max(g n^2 / h^(1/3), Cf); |u| / h as sqrt(qx^2 + qy^2) / h^2 where the reference has
+            // hypot of the velocities (within a few ulps; momenta are far from hypot's overflow range)
+            if (FRIC) {
+                const Real cf = A.friction == DGSW_FRICTION_MANNING ? manning_cf<Real>(A.manning[d], h, (Real)A.friction_cf)
+                                                                    : (Real)A.friction_cf;
+                const Real tau = cf * sqrt(m.x * m.x + m.y * m.y) * (ih * ih);
+                S12 = fma2<PK, Real>(m, -tau, S12);
+            }
+            // int F . grad(phi) = sum_gp sum_z F . J^-1(z, :) dphi_z w
+            sfor<0, ND>([&](auto K) {
+                constexpr int k = decltype(K)::value;
+                auto slope = [&](Two<Real> c) {  // the source, whose continuity part only an analytic source has
+                    if constexpr (FSRC) {
+                        add_to(k, S0, S12, c);
+                    } else {
+                        const Two<Real> r = fma2<PK, Real>(S12, c, Two<Real>{rhs[1][k], rhs[2][k]});
+                        rhs[1][k] = r.x, rhs[2][k] = r.y;
+                    }
+                };
+                if constexpr (ROLL_V) {
+                    if constexpr (counts_any<P>(1, k)) add_to(k, U0, G0, pair_of(TB.m0[gp][k]));
+                    if constexpr (counts_any<P>(2, k)) add_to(k, U1, G1, pair_of(TB.m1[gp][k]));
+                    if constexpr (counts_any<P>(3, k)) slope(pair_of(TB.pw[gp][k]));
+                } else {
+                    constexpr int i = decltype(GP)::value;
+                    constexpr double m0 = MT<P>::mz((0 * NQ + i) * ND + k);
+                    constexpr double m1 = MT<P>::mz((1 * NQ + i) * ND + k);
+                    constexpr double pw = MT<P>::phiw(i * ND + k);
+                    if constexpr (counts(m0)) add_to(k, U0, G0, both(m0));
+                    if constexpr (counts(m1)) add_to(k, U1, G1, both(m1));
+                    if constexpr (counts(pw)) slope(both(pw));
+                }
+            });
+        };
+        if constexpr (ROLL_V) {
+#pragma unroll 1
+            for (int gp = 0; gp < NQ; ++gp) volume_point(gp);
+        } else {
+            sfor<0, NQ>(volume_point);
         }
+        // analytic source_q(t, x_gp) (swe_source.hpp:9-14), in a loop of its own so that its temporaries are not
+        // live together with the flux computation's
+        // The manufactured sine set in FP64 on elements small against its wavelength (k times the
+        // largest vertex offset from the centroid <= 0.05): sin and cos once at the centroid, turned to
+        // each quadrature point by rotate_small; the point's offset from the centroid is
+        // sum_i (psi_i - 1/3) (x_i - x_0), its coordinate never formed. Measured on 524,288 triangles at
+        // p = 2: FP64 stage 212 -> 201 us; in FP32 the hardware sine/cosine per point stays cheaper
+        // (114 against 116 us).
+        const double xc = (x0 + x1 + x2) * (1.0 / 3.0), yc = (y0 + y1 + y2) * (1.0 / 3.0);
+        bool near = false;
+        if constexpr (sizeof(Real) == 8)
+            near = sine_set && (double)SS.k * fmax(fmax(fmax(fabs(x0 - xc), fabs(x1 - xc)), fabs(x2 - xc)),
+                                                     fmax(fmax(fabs(y0 - yc), fabs(y1 - yc)), fabs(y2 - yc))) <= 0.05;
+        if constexpr (sizeof(Real) == 8) {
+            if (FSRC && near) {
+                double sxc, cxc, syc, cyc;
+                sine_src_sincos<Real>(SS, xc, sxc, cxc);
+                sine_src_sincos<Real>(SS, yc, syc, cyc);
+                const double ex1 = x1 - x0, ex2 = x2 - x0, ey1 = y1 - y0, ey2 = y2 - y0;
+                auto near_point = [&](auto GP) {
+                    const auto gp = GP;
+                    const int i = gp;
+                    const double a1 = TB.psi[i][1] - 1.0 / 3.0, a2 = TB.psi[i][2] - 1.0 / 3.0;
+                    double sx, cx, sy, cy;
+                    rotate_small(sxc, cxc, SS.k * (ex1 * a1 + ex2 * a2), sx, cx);
+                    rotate_small(syc, cyc, SS.k * (ey1 * a1 + ey2 * a2), sy, cy);
+                    Real f0;
+                    Two<Real> f12;
+                    sine_src_terms<PK, Real>(SS, sx, cx, sy, cy, f0, f12);
+                    sfor<0, ND>([&](auto K) {
+                        constexpr int k = decltype(K)::value;
+                        if constexpr (ROLL_V) {
+                            if constexpr (counts_any<P>(3, k)) add_to(k, f0, f12, pair_of(TB.pw[gp][k]));
+                        } else {
+                            constexpr double pw = MT<P>::phiw(decltype(GP)::value * ND + k);
+                            if constexpr (counts(pw)) add_to(k, f0, f12, both(pw));
+                        }
+                    });
+                };
+                if constexpr (ROLL_V) {
+#pragma unroll 1
+                    for (int gp = 0; gp < NQ; ++gp) near_point(gp);
+                } else {
+                    sfor<0, NQ>(near_point);
+                }
+            }
+        }
+        if (FSRC && !near && !(sizeof(Real) == 4 && sine_set)) {
+            const Real xr0 = (Real)x0, xr1 = (Real)x1, xr2 = (Real)x2;
+            const Real yr0 = (Real)y0, yr1 = (Real)y1, yr2 = (Real)y2;
+#pragma unroll 1
+            for (int gp = 0; gp < NQ; ++gp) {
+                // FP32 path: Gauss-point coordinates in FP32 (the analytic source is evaluated in FP32)
+                const Real xg = xr0 * TB.psi[gp][0] + xr1 * TB.psi[gp][1] + xr2 * TB.psi[gp][2];
+                const Real yg = yr0 * TB.psi[gp][0] + yr1 * TB.psi[gp][1] + yr2 * TB.psi[gp][2];
+                Val3<Real> r;
+                if (sine_set)
+                    // FP64 elements large against the wavelength: out of line, so that this rarely
+                    // taken path keeps the kernel's hot code small
+                    r = sine_src_far<Real>(&ST, xg, yg);
+                else
+                    r = fn_eval_dev<Real>(A.fn_set, A.fn_params, &FT, 1, xg, yg);
+                sfor<0, ND>([&](auto K) {
+                    constexpr int k = decltype(K)::value;
+                    if constexpr (counts_any<P>(3, k)) add_to(k, r.v0, Two<Real>{r.v1, r.v2}, pair_of(TB.pw[gp][k]));
+                });
+            }
+        }
+        // the volume integrals stay in master-element units: sol = (|J| V + E) M^-1 / |J| is computed as
+        // V M^-1 + (E / |J|) M^-1, with 1 / |J| in the faces' weights
     }
     double comb[3][ND];
     double bv[3] = {0.0, 0.0, 0.0};
-    // phase 3's global loads: the RK combination's state terms and the wet/dry vertex depths, issued when
-    // phase 3 starts (issuing them before the CTA's second barrier instead gained nothing, measured on the
-    // p = 1 and p = 2 workloads in both precisions)
-    auto load_phase3 = [&]() {
+    // the loads of the CTA's end: the RK combination's state terms and the wet/dry vertex depths, issued ahead
+    // of the face loop
+    auto load_end = [&]() {
         if constexpr (SPLIT) split_comb();
 #pragma unroll
         for (int v = 0; v < 3; ++v)
@@ -1491,127 +1568,170 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
                 for (int k = 0; k < ND; ++k) comb[v][k] += aj * t[v][k];
         }
         // wetting/drying: the element's vertex depths, loaded now (two dependent loads) so that their latency
-        // overlaps the edge gather instead of opening the wet/dry pass
+        // overlaps the face loop instead of opening the wet/dry pass
         if (WD) {
             const int n0 = A.enodes[d], n1 = A.enodes[P_ + d], n2 = A.enodes[2 * P_ + d];
             bv[0] = A.nz[n0], bv[1] = A.nz[n1], bv[2] = A.nz[n2];
         }
     };
-    __syncthreads();
-
-    // ---------------- phase 3: edge contributions, M^-1, RK combination, wet/dry ----------------
+    if (!stage_bar_wait(&bar)) {
+        if (tid == 0) atomicOr(&A.status->wait_failed, 1u);
+        return;
+    }
     if (!active) return;
+
+    // ---------------- face fluxes and lift, M^-1, RK combination, wet/dry ----------------
     // the RK combination's state terms, sum_j a_j q_j + dt b_j sol_j over the earlier stages plus
     // a_s q_s, in FP64: all loads of one term are issued together here so that their latency overlaps
-    // the edge gather below (one dependent load per value at the end of the CTA cost a global-memory
+    // the face loop below (one dependent load per value at the end of the CTA cost a global-memory
     // latency per value, per wave)
-    load_phase3();
-    const Real iaJ = Real(1) / aJ;
-    const int roles = es.y & 7;
-    const int ord = es.y >> 3;
-    const int cnt = ord & 3;
-#pragma unroll 1
-    for (int i = 0; i < cnt; ++i) {
-        const int f = (ord >> (2 + 2 * i)) & 3;
-        const int slot = (es.x >> (10 * f)) & 1023;
-        const int sfl = sflag[slot];
-        if (!sfl) continue;
-        const bool is_in = (roles >> f) & 1;
-        const Real sJe = ssJ[slot] * iaJ;  // edge half length over |J|
-        Real F[3][NG];
+    if constexpr (!fw_early) {
 #pragma unroll
-        for (int gp = 0; gp < NG; ++gp) {  // own Gauss point order
-            if (is_in) {
-#pragma unroll
-                for (int v = 0; v < 3; ++v) F[v][gp] = sF[(v * NG + gp) * max_edges + slot];
-            } else if (sfl == 2) {  // levee ex side: its own flux, left in its face's trace slot
-#pragma unroll
-                for (int v = 0; v < 3; ++v) F[v][gp] = tr_at(v, NG - 1 - gp, 3 * tid + f);
+        for (int f = 0; f < 3; ++f) fw[f] = A.fw[f * P_ + d];
+    }
+    load_end();
+    // the faces' lift, rhs += T phi_k(gp) on face f
+    auto lift = [&](auto FF, auto GP, Real T0, Two<Real> T12) {
+        const auto fc = FF;
+        const auto gc = GP;
+        const int f = fc, gp = gc;
+        sfor<0, ND>([&](auto K) {
+            constexpr int k = decltype(K)::value;
+            if constexpr (std::is_same<decltype(FF), int>::value) {
+                if constexpr (counts_any<P>(4, k)) add_to(k, T0, T12, pair_of(TB.fphi[f][gp][k]));
             } else {
-                const int ga = NG - 1 - gp;
-#pragma unroll
-                for (int v = 0; v < 3; ++v)
-                    F[v][gp] = WD ? sF[((3 + v) * NG + ga) * max_edges + slot] : -sF[(v * NG + ga) * max_edges + slot];
+                constexpr double c = MT<P>::fphi((decltype(FF)::value * ND + k) * NG + decltype(GP)::value);
+                if constexpr (counts(c)) add_to(k, T0, T12, both(c));
             }
-        }
-        if constexpr (rt_face) {
-            // rhs -= sum_gp F phi_k w |e|/2 / |J| with the face's basis values from shared memory (a value
-            // that is zero on this face but not on another subtracts a zero product: the sum is unchanged)
-            const Real* __restrict__ cf = sfphi + f * ND * NG;
+        });
+    };
+    // on: a face between wet elements, or a boundary face of one; these run without branches, so that one face's
+    // loads overlap another's arithmetic. special: an interface with one dry side, a levee, the spherical correction;
+    // few elements have one, and a rolled loop takes them afterwards.
+    bool on[3];
+    int special = 0;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+        const int kind = meta[f] & 7;
+        const bool wn = kind >= 5 ? wet : swet[meta[f] >> 4] != 0;
+        const bool any = kind < 5 && (wet || wn);
+        const bool sp = kind == 5 || (any && ((WD && wet != wn) || A.spherical));
+        on[f] = any && !sp;
+        if (sp) special |= 1 << f;
+    }
+    if (!WD || on[0] || on[1] || on[2]) {
+        auto face = [&](auto FF) {
+            const auto fc = FF;  // IC<f> (unrolled) or an int
+            const int f = fc;
+            const Two<Real> N = scaled_normal<Real>(f, Ji00, Ji01, Ji10, Ji11);
+            const int m = f == 0 ? meta[0] : (f == 1 ? meta[1] : meta[2]);
+            const Real w = f == 0 ? fw[0] : (f == 1 ? fw[1] : fw[2]);
+            const bool o_f = f == 0 ? on[0] : (f == 1 ? on[1] : on[2]);
+            const int slot = o_f ? m >> 4 : 3 * tid + f;  // a levee's payload is no slot
             sfor<0, NG>([&](auto GP) {
                 constexpr int gp = decltype(GP)::value;
-                const Real wsJ = (Real)MT<P>::gw(gp) * sJe;
-                Real T[3];
-#pragma unroll
-                for (int v = 0; v < 3; ++v) T[v] = F[v][gp] * wsJ;
-                sfor<0, ND>([&](auto K) {
-                    constexpr int k = decltype(K)::value;
-                    constexpr bool used = MT<P>::fphi((0 * ND + k) * NG + gp) != 0.0 ||
-                                          MT<P>::fphi((1 * ND + k) * NG + gp) != 0.0 ||
-                                          MT<P>::fphi((2 * ND + k) * NG + gp) != 0.0;
-                    if constexpr (used) {
-                        const Real c = cf[k * NG + gp];
-                        if constexpr (packed) {
-                            // packed FP32: ze and qx share the coefficient (qy alone), as fma(-T, c, rhs)
-                            fma_pair(rhs[0][k], rhs[1][k], -T[0], -T[1], c, c);
-                            rhs[2][k] = __fmaf_rn(-T[2], c, rhs[2][k]);
-                        } else {
-#pragma unroll
-                            for (int v = 0; v < 3; ++v) rhs[v][k] -= T[v] * c;
-                        }
-                    }
-                });
+                const Side<Real> o = TR::get(tr, NS, 3 * tid + f, gp, g);
+                const Side<Real> n = TR::get(tr, NS, slot, NG - 1 - gp, g);
+                Real F0;
+                Two<Real> F12;
+                llf_sides<PK, Real>(g, o, n, N, w, F0, F12);
+                // rhs -= F phi_k w |e|/2 / |J|; the flux's 1/2 is in the weight, |e|/2 / |J| in the flux
+                const Real wg = (Real)(-0.5 * MT<P>::gw(gp));
+                const Two<Real> T12 = mul2<PK, Real>(F12, wg);
+                lift(FF, GP, o_f ? F0 * wg : Real(0), Two<Real>{o_f ? T12.x : Real(0), o_f ? T12.y : Real(0)});
             });
+        };
+        if constexpr (ROLL_F) {
+#pragma unroll 1
+            for (int f = 0; f < 3; ++f) face(f);
         } else {
-            auto contrib = [&](auto FF) {
-                constexpr int fc = decltype(FF)::value;
-                sfor<0, NG>([&](auto GP) {
-                    constexpr int gp = decltype(GP)::value;
-                    const Real wsJ = (Real)MT<P>::gw(gp) * sJe;
-                    Real T[3];
-#pragma unroll
-                    for (int v = 0; v < 3; ++v) T[v] = F[v][gp] * wsJ;
-                    sfor<0, ND>([&](auto K) {
-                        constexpr int k = decltype(K)::value;
-                        constexpr double c = MT<P>::fphi((fc * ND + k) * NG + gp);
-                        if constexpr (c != 0.0) {
-                            if constexpr (packed) {
-                                // packed FP32: ze and qx share the coefficient (qy alone), as fma(-T, c, rhs)
-                                fma_pair(rhs[0][k], rhs[1][k], -T[0], -T[1], (Real)c, (Real)c);
-                                rhs[2][k] = __fmaf_rn(-T[2], (Real)c, rhs[2][k]);
-                            } else {
-#pragma unroll
-                                for (int v = 0; v < 3; ++v) rhs[v][k] -= T[v] * (Real)c;
+            sfor<0, 3>(face);
+        }
+    }
+    if (special) {
+#pragma unroll 1
+        for (int f = 0; f < 3; ++f) {
+            if (!(special >> f & 1)) continue;
+            const int fm = A.fmeta[f * P_ + d];
+            const Real w = A.fw[f * P_ + d];
+            const int kind = fm & 7;
+            const bool is_in = fm & 8;
+            if (kind == 5) {  // a levee interface's flux comes from levee.cu
+                const double* Fl = A.levF + (size_t)(fm >> 4) * (6 * NG);
+#pragma unroll 1
+                for (int gp = 0; gp < NG; ++gp) {
+                    const int at = is_in ? gp : 3 * NG + NG - 1 - gp;
+                    const Real wg = -TB.gw[gp] * w;
+                    lift(f, gp, (Real)Fl[at] * wg, Two<Real>{(Real)Fl[NG + at] * wg, (Real)Fl[2 * NG + at] * wg});
+                }
+                continue;
+            }
+            const int slot = fm >> 4;
+            const bool wn = swet[slot] != 0;
+            const Two<Real> N = scaled_normal<Real>(f, Ji00, Ji01, Ji10, Ji11);
+            const Real iw = Real(1) / w, thr = Real(2e-12) * w;
+#pragma unroll 1
+            for (int gp = 0; gp < NG; ++gp) {
+                Side<Real> o = TR::get(tr, NS, 3 * tid + f, gp, g);
+                Side<Real> n = TR::get(tr, NS, slot, NG - 1 - gp, g);
+                if (WD && sizeof(Real) == 8) {  // a dry side's trace comes without them
+                    if (!wet) complete<Real>(o, g);
+                    if (!wn) complete<Real>(n, g);
+                }
+                Real F0;
+                Two<Real> F12;
+                if (A.spherical) {
+                    Val3<Real> r = spherical_flux<P, Real>(&A, d, f, gp, is_in, o.ze, o.q.x, o.q.y, o.b, n.ze, n.q.x, n.q.y,
+                                                           n.b, N.x, N.y, w);
+                    if (WD && wet != wn)
+                        r = wd_fixup_own<P, Real>(&A, d, f, gp, is_in, wet, wn, o.ze, o.q.x, o.q.y, o.b, n.ze, n.q.x, n.q.y,
+                                                  n.b, N.x, N.y, w, r.v0, r.v1, r.v2);
+                    F0 = r.v0, F12 = {r.v1, r.v2};
+                } else {
+                    llf_sides<PK, Real>(g, o, n, N, w, F0, F12);
+                    if (WD && wet != wn) {
+                        // the fix-ups of wd_fixup (rkdg_swe_is_internal.hpp:47-90) as the own side sees them
+                        if (F0 > thr) {
+                            if (!wet) F0 = Real(0), F12 = {Real(0), Real(0)};  // none leaves a dry element
+                        } else if (F0 < -thr) {
+                            if (!wn) {  // none comes from a dry neighbour: a reflective wall
+                                // the mirrored state's flux in closed form: no mass through the wall, and twice the
+                                // pressure and the normal momentum's upwinding on it
+                                const Real fo = fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)), uo = fo * o.ih;
+                                const Real a = (uo + fabs(uo) + o.c * w) * (2 * fo * iw * iw) +
+                                               2 * (g * o.ze * (Real(0.5) * o.ze + o.b));
+                                F0 = Real(0), F12 = {a * N.x, a * N.y};
+                            } else {  // into a dry element: gravity-free momentum flux
+                                o.c = n.c = Real(0);
+                                Real F0g;
+                                llf_sides<PK, Real>(Real(0), o, n, N, w, F0g, F12);
                             }
                         }
-                    });
-                });
-            };
-            if (f == 0)
-                contrib(IC<0>{});
-            else if (f == 1)
-                contrib(IC<1>{});
-            else
-                contrib(IC<2>{});
+                    }
+                }
+                const Real wg = Real(-0.5) * TB.gw[gp];
+                lift(f, gp, F0 * wg, mul2<PK, Real>(F12, wg));
+            }
         }
     }
     // M^-1 (the diagonal master mass inverse; 1 / |J| is already in) and the SSP-RK stage combination
     const double bdt_s = A.bdt[A.nterms - 1];
     if constexpr (SPLIT) {
         const Real bs = (Real)bdt_s;
-        // dn = dcomb + dt b_s (rhs M^-1), ze and qx packed (each lane the scalar mul and fma)
+        // dn = dcomb + dt b_s (rhs M^-1), qx and qy packed (each lane the scalar mul and fma)
         Real (&dn)[3][ND] = dcomb;
         sfor<0, ND>([&](auto K) {
             constexpr int k = decltype(K)::value;
             const Real mk = (Real)MT<P>::minv(k);
-            const float2 s01 = __fmul2_rn(make_float2(rhs[0][k], rhs[1][k]), make_float2(mk, mk));
-            const Real sol[3] = {s01.x, s01.y, rhs[2][k] * mk};
+            const Two<Real> s12 = mul2<PK, Real>(Two<Real>{rhs[1][k], rhs[2][k]}, mk);
+            const Real sol[3] = {mul_rn(rhs[0][k], mk), s12.x, s12.y};
             if (A.store_sol) {
 #pragma unroll
                 for (int v = 0; v < 3; ++v) A.dsol_out[(v * ND + k) * P_ + d] = sol[v];
             }
-            fma_pair(dn[0][k], dn[1][k], sol[0], sol[1], bs, bs);
-            dn[2][k] = __fmaf_rn(sol[2], bs, dn[2][k]);
+            const Two<Real> r = fma2<PK, Real>(s12, bs, Two<Real>{dn[1][k], dn[2][k]});
+            dn[1][k] = r.x, dn[2][k] = r.y;
+            dn[0][k] = fma_rn(sol[0], bs, dn[0][k]);
         });
         bool has_nan = false;
         if (A.last) {
@@ -1705,64 +1825,58 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, OCC>::valu
 constexpr int STAGE_MODE_OCC = 8;
 // bit 4 of `mode`: the kernel with run-time shared-memory strides even where the mesh fits the caps
 constexpr int STAGE_MODE_UNCAPPED = 16;
-cudaError_t launch_stage_p1_f64(const StageArgs<double>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p1_f64(const StageArgs<double>& A, int tile, int ntiles, int max_halo,
                                 int mode, cudaStream_t s);
-cudaError_t launch_stage_p1_f32(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p1_f32(const StageArgs<float>& A, int tile, int ntiles, int max_halo,
                                 int mode, cudaStream_t s);
-cudaError_t launch_stage_p2_f64(const StageArgs<double>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p2_f64(const StageArgs<double>& A, int tile, int ntiles, int max_halo,
                                 int mode, cudaStream_t s);
-cudaError_t launch_stage_p2_f32(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p2_f32(const StageArgs<float>& A, int tile, int ntiles, int max_halo,
                                 int mode, cudaStream_t s);
-cudaError_t launch_stage_p1_f64_occ(const StageArgs<double>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p1_f64_occ(const StageArgs<double>& A, int tile, int ntiles, int max_halo,
                                     int mode, cudaStream_t s);
-cudaError_t launch_stage_p1_f32_occ(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p1_f32_occ(const StageArgs<float>& A, int tile, int ntiles, int max_halo,
                                     int mode, cudaStream_t s);
-cudaError_t launch_stage_p2_f64_occ(const StageArgs<double>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p2_f64_occ(const StageArgs<double>& A, int tile, int ntiles, int max_halo,
                                     int mode, cudaStream_t s);
-cudaError_t launch_stage_p2_f32_occ(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p2_f32_occ(const StageArgs<float>& A, int tile, int ntiles, int max_halo,
                                     int mode, cudaStream_t s);
 // stage increments (StageArgs::dk ...): the default budget, or the alternative one with bit 3 of `mode`
-cudaError_t launch_stage_p1_f32_split(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p1_f32_split(const StageArgs<float>& A, int tile, int ntiles, int max_halo,
                                       int mode, cudaStream_t s);
-cudaError_t launch_stage_p2_f32_split(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_p2_f32_split(const StageArgs<float>& A, int tile, int ntiles, int max_halo,
                                       int mode, cudaStream_t s);
 
-// whether every tile of a mesh fits the compile-time shared-memory capacities of the capped kernels
-inline bool stage_fits_caps(int tile, int max_halo, int max_edges) {
-    return tile == 128 ? max_halo <= TileCap<128>::halo && max_edges <= TileCap<128>::edges
-                       : max_halo <= TileCap<256>::halo && max_edges <= TileCap<256>::edges;
+// whether every tile of a mesh fits the compile-time shared-memory capacity of the capped kernels
+inline bool stage_fits_caps(int tile, int max_halo) {
+    return max_halo <= (tile == 128 ? TileCap<128>::halo : TileCap<256>::halo);
 }
 
 // with `allow_capped` false the kernel with run-time strides runs even where the mesh fits the caps: its
 // shared memory is sized to the mesh's largest tile, and with less shared memory per SM the L1 cache that
 // shares its storage is larger (the autotuner times both)
 template <int P, typename Real, bool WD, bool FSRC, bool FRIC, int TILE, int OCC, bool SPLIT = false>
-cudaError_t launch_stage_impl(const StageArgs<Real>& A, int ntiles, int max_halo, int max_edges, bool allow_capped,
-                              cudaStream_t s) {
-    const bool capped = allow_capped && max_halo <= TileCap<TILE>::halo && max_edges <= TileCap<TILE>::edges;
+cudaError_t launch_stage_impl(const StageArgs<Real>& A, int ntiles, int max_halo, bool allow_capped, cudaStream_t s) {
+    const bool capped = allow_capped && max_halo <= TileCap<TILE>::halo;
     auto kern = capped ? rkdg_stage_kernel<P, Real, WD, FSRC, FRIC, TILE, true, OCC, SPLIT>
                        : rkdg_stage_kernel<P, Real, WD, FSRC, FRIC, TILE, false, OCC, SPLIT>;
     // the run-time-stride kernel loads its halo faces' elements straight from global memory and never
     // touches the halo staging area (every use of it is under CAPPED), so its allocation ends there
-    const size_t smem = capped ? Smem<P, Real, WD>::bytes(TILE, TileCap<TILE>::halo, TileCap<TILE>::edges)
-                               : Smem<P, Real, WD>::off_halo(TILE, max_halo, max_edges);
+    const size_t smem = capped ? Smem<P, Real>::bytes(TILE, TileCap<TILE>::halo) : Smem<P, Real>::off_halo(TILE, max_halo);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)(ntiles + A.n_time), TILE, smem, s>>>(A, max_halo, max_edges);
+    kern<<<(unsigned)(ntiles + A.n_time), TILE, smem, s>>>(A, max_halo);
     return cudaGetLastError();
 }
 
 template <int P, typename Real, bool WD, bool FSRC, bool FRIC, int OCC, bool SPLIT = false>
-cudaError_t launch_stage_tile(const StageArgs<Real>& A, int tile, int ntiles, int max_halo, int max_edges, int mode,
-                              cudaStream_t s) {
+cudaError_t launch_stage_tile(const StageArgs<Real>& A, int tile, int ntiles, int max_halo, int mode, cudaStream_t s) {
     const bool allow_capped = !(mode & STAGE_MODE_UNCAPPED);
     switch (tile) {
         case 128:
-            return launch_stage_impl<P, Real, WD, FSRC, FRIC, 128, OCC, SPLIT>(A, ntiles, max_halo, max_edges,
-                                                                                allow_capped, s);
+            return launch_stage_impl<P, Real, WD, FSRC, FRIC, 128, OCC, SPLIT>(A, ntiles, max_halo, allow_capped, s);
         case 256:
-            return launch_stage_impl<P, Real, WD, FSRC, FRIC, 256, OCC, SPLIT>(A, ntiles, max_halo, max_edges,
-                                                                                allow_capped, s);
+            return launch_stage_impl<P, Real, WD, FSRC, FRIC, 256, OCC, SPLIT>(A, ntiles, max_halo, allow_capped, s);
         default:
             return cudaErrorInvalidValue;
     }
@@ -1770,30 +1884,30 @@ cudaError_t launch_stage_tile(const StageArgs<Real>& A, int tile, int ntiles, in
 
 // wetting/drying, function source and bottom friction select the instantiation (bit 0, 1, 2 of `mode`)
 template <int P, typename Real, int OCC>
-cudaError_t launch_stage_dispatch(const StageArgs<Real>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_dispatch(const StageArgs<Real>& A, int tile, int ntiles, int max_halo,
                                   int mode, cudaStream_t s) {
     switch (mode & 7) {
-        case 0: return launch_stage_tile<P, Real, false, false, false, OCC>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 1: return launch_stage_tile<P, Real, true, false, false, OCC>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 2: return launch_stage_tile<P, Real, false, true, false, OCC>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 3: return launch_stage_tile<P, Real, true, true, false, OCC>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 4: return launch_stage_tile<P, Real, false, false, true, OCC>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 5: return launch_stage_tile<P, Real, true, false, true, OCC>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 6: return launch_stage_tile<P, Real, false, true, true, OCC>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        default: return launch_stage_tile<P, Real, true, true, true, OCC>(A, tile, ntiles, max_halo, max_edges, mode, s);
+        case 0: return launch_stage_tile<P, Real, false, false, false, OCC>(A, tile, ntiles, max_halo, mode, s);
+        case 1: return launch_stage_tile<P, Real, true, false, false, OCC>(A, tile, ntiles, max_halo, mode, s);
+        case 2: return launch_stage_tile<P, Real, false, true, false, OCC>(A, tile, ntiles, max_halo, mode, s);
+        case 3: return launch_stage_tile<P, Real, true, true, false, OCC>(A, tile, ntiles, max_halo, mode, s);
+        case 4: return launch_stage_tile<P, Real, false, false, true, OCC>(A, tile, ntiles, max_halo, mode, s);
+        case 5: return launch_stage_tile<P, Real, true, false, true, OCC>(A, tile, ntiles, max_halo, mode, s);
+        case 6: return launch_stage_tile<P, Real, false, true, true, OCC>(A, tile, ntiles, max_halo, mode, s);
+        default: return launch_stage_tile<P, Real, true, true, true, OCC>(A, tile, ntiles, max_halo, mode, s);
     }
 }
 
 // the stage-increment kernels (FP32, no wetting/drying): function source and bottom friction select the
 // instantiation (bits 1 and 2 of `mode`; bit 0, wetting/drying, must be clear)
 template <int P, int OCC>
-cudaError_t launch_stage_split_dispatch(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
+cudaError_t launch_stage_split_dispatch(const StageArgs<float>& A, int tile, int ntiles, int max_halo,
                                         int mode, cudaStream_t s) {
     switch (mode & 7) {
-        case 0: return launch_stage_tile<P, float, false, false, false, OCC, true>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 2: return launch_stage_tile<P, float, false, true, false, OCC, true>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 4: return launch_stage_tile<P, float, false, false, true, OCC, true>(A, tile, ntiles, max_halo, max_edges, mode, s);
-        case 6: return launch_stage_tile<P, float, false, true, true, OCC, true>(A, tile, ntiles, max_halo, max_edges, mode, s);
+        case 0: return launch_stage_tile<P, float, false, false, false, OCC, true>(A, tile, ntiles, max_halo, mode, s);
+        case 2: return launch_stage_tile<P, float, false, true, false, OCC, true>(A, tile, ntiles, max_halo, mode, s);
+        case 4: return launch_stage_tile<P, float, false, false, true, OCC, true>(A, tile, ntiles, max_halo, mode, s);
+        case 6: return launch_stage_tile<P, float, false, true, true, OCC, true>(A, tile, ntiles, max_halo, mode, s);
         default: return cudaErrorInvalidValue;
     }
 }

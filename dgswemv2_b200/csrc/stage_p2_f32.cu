@@ -3,8 +3,8 @@
 #include "stage_kernel.cuh"
 
 namespace dgsw {
-cudaError_t launch_stage_p2_f32(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
-                                int mode, cudaStream_t s) {
-    return launch_stage_dispatch<2, float, 0>(A, tile, ntiles, max_halo, max_edges, mode, s);
+cudaError_t launch_stage_p2_f32(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int mode,
+                                cudaStream_t s) {
+    return launch_stage_dispatch<2, float, 0>(A, tile, ntiles, max_halo, mode, s);
 }
 }  // namespace dgsw

@@ -4,9 +4,9 @@
 #include "stage_kernel.cuh"
 
 namespace dgsw {
-cudaError_t launch_stage_p2_f32_split(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int max_edges,
-                                      int mode, cudaStream_t s) {
-    if (mode & STAGE_MODE_OCC) return launch_stage_split_dispatch<2, 1>(A, tile, ntiles, max_halo, max_edges, mode, s);
-    return launch_stage_split_dispatch<2, 0>(A, tile, ntiles, max_halo, max_edges, mode, s);
+cudaError_t launch_stage_p2_f32_split(const StageArgs<float>& A, int tile, int ntiles, int max_halo, int mode,
+                                cudaStream_t s) {
+    if (mode & STAGE_MODE_OCC) return launch_stage_split_dispatch<2, 1>(A, tile, ntiles, max_halo, mode, s);
+    return launch_stage_split_dispatch<2, 0>(A, tile, ntiles, max_halo, mode, s);
 }
 }  // namespace dgsw

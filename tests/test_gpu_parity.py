@@ -610,3 +610,21 @@ def test_p2_limiter_matches_where_decisions_are_clear(oracle):
         assert np.array_equal(lg, lo)
         assert rel_err(P.get_state(), O.get_state()) <= 1e-12
     assert lo.sum() > 10
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (9, 7), (8, 8), (13, 5), (64, 2)])
+@pytest.mark.parametrize("p,tile", [(1, 128), (1, 256), (2, 128), (2, 256)])
+def test_tile_edges_and_remainders(oracle, nx, ny, p, tile):
+    """Meshes of 2, 126, 128, 130 and 256 triangles (less than a tile, one exactly, a remainder of two, a strip
+    whose tiles are mostly halo and boundary faces) with tide, river and land faces, and stage and step calls mixed:
+    the last element's face slots, the ghost slots behind the halo slots and the forcing values of the second
+    copy of the step's time. Bar: 1e-12 of each variable's scale, as for the other FP64 runs here."""
+    mesh, cfg = configs.tidal_channel(nx, ny, p=p, rk=(2, 2) if p == 1 else (3, 3), dt=0.5, jitter=0.1 if nx > 1 else 0.0)
+    P = Problem(cfg, mesh, tile=tile)
+    O = oracle.problem(cfg, mesh)
+    P.step_serial(3)
+    for _ in range(cfg.rk_nstages):
+        P.stage_serial()
+    P.step_serial(9)
+    O.step(13)
+    assert rel_err(P.get_state(), O.get_state()) <= 1e-12
