@@ -622,6 +622,10 @@ def test_tile_edges_and_remainders(oracle, nx, ny, p, tile):
     mesh, cfg = configs.tidal_channel(nx, ny, p=p, rk=(2, 2) if p == 1 else (3, 3), dt=0.5, jitter=0.1 if nx > 1 else 0.0)
     P = Problem(cfg, mesh, tile=tile)
     O = oracle.problem(cfg, mesh)
+    q = np.random.default_rng(5).uniform(-0.02, 0.02, (P.ne, 3, P.nd))  # every variable well above rounding
+    q[:, 1:] *= 10.0
+    P.set_state(q)
+    O.set_state(q)
     P.step_serial(3)
     for _ in range(cfg.rk_nstages):
         P.stage_serial()
