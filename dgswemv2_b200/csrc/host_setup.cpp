@@ -389,7 +389,6 @@ int build_topology(const dgsw_mesh* m, Topology& T, std::string& err) {
     // interfaces in (in, ex) order, in = smaller reference ID (swe_pre_create_intface.hpp:14-34): the
     // internal ones, then the levee ones (ProblemInterfaceTypes order)
     T.intf.clear();
-    std::vector<int32_t> intf_of_face(3 * ne, -1);
     {
         // counts per element, prefix sums, then each element writes its own interfaces in place
         std::vector<int32_t> cnt(2 * ne + 1, 0);
@@ -421,44 +420,20 @@ int build_topology(const dgsw_mesh* m, Topology& T, std::string& err) {
                     T.intf[4 * (size_t)idx + 1] = e;
                     T.intf[4 * (size_t)idx + 2] = f;
                     T.intf[4 * (size_t)idx + 3] = fe;
-                    intf_of_face[3 * r + f] = idx;
-                    intf_of_face[3 * (int64_t)e + fe] = idx;
                 }
             }
         }
     }
     // boundaries grouped by type (Land, Tide, Flow, Function tuple order), each by (element, face)
     T.bnd.clear();
-    std::vector<int64_t> bnd_of_face(3 * ne, -1);
     for (int bt : {DGSW_BC_LAND, DGSW_BC_TIDE, DGSW_BC_FLOW, DGSW_BC_FUNCTION}) {
         for (int64_t r = 0; r < ne; ++r)
             for (int f = 0; f < 3; ++f)
                 if (T.btype[3 * r + f] == bt) {
-                    bnd_of_face[3 * r + f] = (int64_t)T.bnd.size() / 3;
                     T.bnd.push_back((int32_t)r);
                     T.bnd.push_back(f);
                     T.bnd.push_back(bt);
                 }
-    }
-    // per element accumulation order: its interfaces by creation index, then its boundaries
-    T.order_count.assign(ne, 0);
-    T.order_face.assign(3 * ne, 0);
-    T.is_in.assign(3 * ne, 0);
-#pragma omp parallel for schedule(static)
-    for (int64_t r = 0; r < ne; ++r) {
-        std::pair<int64_t, int> items[3];
-        int n = 0;
-        for (int f = 0; f < 3; ++f)
-            if (intf_of_face[3 * r + f] >= 0) items[n++] = {intf_of_face[3 * r + f], f};
-        std::sort(items, items + n);
-        int ni = n;
-        for (int f = 0; f < 3; ++f)
-            if (bnd_of_face[3 * r + f] >= 0) items[n++] = {bnd_of_face[3 * r + f], f};
-        std::sort(items + ni, items + n);
-        T.order_count[r] = (uint8_t)n;
-        for (int k = 0; k < n; ++k) T.order_face[3 * r + k] = (uint8_t)items[k].second;
-        // the element owns the flux evaluation of its boundary faces and of interfaces to larger IDs
-        for (int f = 0; f < 3; ++f) T.is_in[3 * r + f] = (T.nbr[3 * r + f] > r || T.nbr[3 * r + f] < 0) ? 1 : 0;
     }
     return DGSW_OK;
 }

@@ -55,10 +55,6 @@ struct Topology {
     bigvec<int32_t> intf;           // [4*n_intf] in, ex, face_in, face_ex in creation order
     int64_t n_intf_internal = 0;    // the internal interfaces come first, then the levee ones
     std::vector<int32_t> bnd;       // [3*n_bnd] elem, face, type in traversal order
-    // per element: faces in accumulation order (interfaces by creation order, then boundaries)
-    std::vector<uint8_t> order_count;  // [ne]
-    std::vector<uint8_t> order_face;   // [3*ne]
-    std::vector<uint8_t> is_in;        // [3*ne] element is the "in" side of the interface on this face
     // ensembles: member of element r (empty for a single problem) and each member's function-set
     // parameters [n_members][DGSW_FN_PARAMS]
     std::vector<int32_t> group;
