@@ -219,6 +219,7 @@ SIGNATURES = {
                                   C.c_int64, C.c_void_p, C.c_void_p]),
     "dgsw_mlp_adam": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_float, C.c_float,
                                   C.c_float, C.c_float, C.c_void_p]),
+    "dgsw_check_stage_barrier": (C.c_int32, [C.c_void_p, C.c_uint32, C.c_uint32, C.POINTER(C.c_uint32)]),
     "dgsw_check_llf_flux": (C.c_int32, [C.c_int32, C.c_int64, C.c_double] + [C.POINTER(C.c_double)] * 6),
     "dgsw_check_internal_flux": (C.c_int32, [C.c_int32, C.c_int64, C.c_double] + [C.POINTER(C.c_double)] * 6 +
                                  [C.POINTER(C.c_uint8)] * 2 + [C.POINTER(C.c_double)] * 2),

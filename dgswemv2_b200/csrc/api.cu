@@ -77,6 +77,25 @@ int make_l2_rule(L2Rule& R, std::string& err) {
 
 __global__ void step_time_kernel(const __grid_constant__ TimeArgs T) { form_step_time(&T, (int)blockIdx.x); }
 
+// the stage kernel's barrier with chosen warps late: they arrive once the others' waits have ended, either way
+__global__ void __launch_bounds__(128) check_barrier_kernel(unsigned late, unsigned polls, DevStatus* status,
+                                                            unsigned* gave_up) {
+    __shared__ unsigned long long bar;
+    const unsigned warp = threadIdx.x / 32;
+    const bool is_late = late >> warp & 1u;
+    if (threadIdx.x == 0) stage_bar_init(&bar, 4);
+    __syncthreads();
+    if (!is_late) {
+        stage_bar_arrive(&bar);
+        if (!stage_bar_wait(&bar, status, polls)) atomicOr(gave_up, 1u << warp);
+    }
+    __syncthreads();
+    if (is_late) {
+        stage_bar_arrive(&bar);
+        if (!stage_bar_wait(&bar, status)) atomicOr(gave_up, 1u << warp);
+    }
+}
+
 }  // namespace
 
 namespace dgsw {
@@ -575,6 +594,13 @@ int check_status(dgsw_rkdg_s* h) {
     DevStatus st;
     CUDA_TRY(cudaMemcpyAsync(&st, h->status.p, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
+    if (st.wait_failed || st.nan_flag) {  // reported once: the next batch starts with a clean record
+        DevStatus z;
+        std::memset(&z, 0, sizeof(z));
+        z.nan_key = ~0ull;
+        cudaMemcpyAsync(h->status.p, &z, sizeof(z), cudaMemcpyHostToDevice, h->stream);
+        cudaStreamSynchronize(h->stream);
+    }
     if (st.wait_failed) return fail(DGSW_ERR_CUDA, "stage kernel: a barrier wait gave up");
     if (st.nan_flag) {
         // the first stage with a NaN and its smallest element, as the reference's per-stage scrutiny
@@ -582,11 +608,6 @@ int check_status(dgsw_rkdg_s* h) {
         const uint32_t ref = (uint32_t)(st.nan_key & 0xffffffffull);
         const unsigned long long counter = st.nan_key >> 32;
         uint32_t id = ref < h->topo.ids.size() ? h->topo.ids[ref] : 0;
-        DevStatus z;
-        std::memset(&z, 0, sizeof(z));
-        z.nan_key = ~0ull;
-        cudaMemcpyAsync(h->status.p, &z, sizeof(z), cudaMemcpyHostToDevice, h->stream);
-        cudaStreamSynchronize(h->stream);
         return fail(DGSW_ERR_NAN, "Fatal Error: NaN found at element " + std::to_string(id) + " (step " +
                                       std::to_string(counter / (unsigned long long)h->ns) + ", stage " +
                                       std::to_string(counter % (unsigned long long)h->ns) + ")");
@@ -1932,6 +1953,24 @@ int32_t dgsw_rkdg_step_timed(dgsw_handle h, int32_t nsteps, double* stage_ms, in
     }
     if (stage_ms) *stage_ms = total;
     if (stage_launches) *stage_launches = (int64_t)(h->kt_used / 2);
+    return DGSW_OK;
+}
+
+int32_t dgsw_check_stage_barrier(dgsw_handle h, uint32_t late_warps, uint32_t polls, uint32_t* gave_up) {
+    if (!h || !gave_up || late_warps > 15u || polls == 0 || polls > STAGE_BAR_POLLS)
+        return fail(DGSW_ERR_INVALID_ARGUMENT, "barrier check: bad arguments");
+    cudaSetDevice(h->device);
+    DBuf<unsigned> d;
+    cudaError_t e = d.alloc(1);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d.p, 0, sizeof(unsigned), h->stream);
+    if (e == cudaSuccess) {
+        check_barrier_kernel<<<1, 128, 0, h->stream>>>(late_warps, polls, h->status.p, d.p);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(gave_up, d.p, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    d.release();
+    if (e != cudaSuccess) return fail(DGSW_ERR_CUDA, std::string("barrier check: ") + cudaGetErrorString(e));
     return DGSW_OK;
 }
 

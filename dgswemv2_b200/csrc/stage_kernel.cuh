@@ -116,7 +116,7 @@ constexpr bool counts(double c) { return c > 1e-13 || c < -1e-13; }
 struct DevStatus {
     unsigned long long nan_key;  // ~0 while no NaN has been seen
     unsigned int nan_flag;
-    unsigned int wait_failed;  // a CTA gave up waiting at its barrier
+    unsigned int wait_failed;  // a thread gave up waiting at its CTA's barrier
 };
 
 constexpr int SINE_NCONST = 10;
@@ -1026,9 +1026,14 @@ __device__ __forceinline__ void stage_bar_arrive(unsigned long long* bar) {
                          (unsigned)__cvta_generic_to_shared(bar))
                      : "memory");
 }
-__device__ __forceinline__ bool stage_bar_wait(unsigned long long* bar) {
+// polls of the bounded wait. All warps of a CTA arrive, so that a wait that runs out means a fault of this code
+constexpr unsigned STAGE_BAR_POLLS = 1u << 24;
+// false, and recorded in the status by whichever thread it happens to, when the wait runs out: its element's results
+// stay unwritten, whatever the other warps' waits do
+__device__ __forceinline__ bool stage_bar_wait(unsigned long long* bar, DevStatus* status,
+                                               unsigned polls = STAGE_BAR_POLLS) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-    for (unsigned i = 0; i < (1u << 24); ++i) {
+    for (unsigned i = 0; i < polls; ++i) {
         unsigned done;
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -1037,6 +1042,7 @@ __device__ __forceinline__ bool stage_bar_wait(unsigned long long* bar) {
             : "memory");
         if (done) return true;
     }
+    atomicOr(&status->wait_failed, 1u);
     return false;
 }
 
@@ -1574,10 +1580,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
             bv[0] = A.nz[n0], bv[1] = A.nz[n1], bv[2] = A.nz[n2];
         }
     };
-    if (!stage_bar_wait(&bar)) {
-        if (tid == 0) atomicOr(&A.status->wait_failed, 1u);
-        return;
-    }
+    if (!stage_bar_wait(&bar, A.status)) return;
     if (!active) return;
 
     // ---------------- face fluxes and lift, M^-1, RK combination, wet/dry ----------------

@@ -6,7 +6,8 @@ self-check entry points run the stage kernel's llf_flux, ISP::Internal fix-ups a
 - wetting/drying: the five single-element cases of test/test_wetting_drying.cpp:15-380
   (tests/golden/wetting_drying.json), within each case's stated tolerance;
 - ISP::Internal::ComputeFlux (rkdg_swe_is_internal.hpp:26-95, no reference unit test): random states on
-  both sides with every wet/dry combination, against the oracle's restatement, FP64 within 1e-13 of the flux scale.
+  both sides with every wet/dry combination, against the oracle's restatement, FP64 within 1e-13 of the flux scale;
+- the stage kernel's bounded barrier wait: a wait that runs out in any warp is reported, once.
 """
 import ctypes as C
 import json
@@ -15,7 +16,7 @@ import os
 import numpy as np
 import pytest
 
-from dgswemv2_b200 import _lib
+from dgswemv2_b200 import DgswError, Problem, _lib, configs
 
 pytestmark = pytest.mark.gpu
 GOLD = os.path.join(os.path.dirname(__file__), "golden")
@@ -135,3 +136,23 @@ def test_internal_flux_with_wet_dry_fixups_against_the_oracle(oracle):
             kinds.add((int(wet_in[k]), int(wet_ex[k]), bool(F[0] > 0)))
     # every branch of the fix-up ran
     assert len(kinds) >= 6, kinds
+
+
+@pytest.mark.parametrize("late", [0, 1, 2, 8, 5, 15])
+def test_a_barrier_wait_that_runs_out_is_reported_once(late):
+    """Warps that arrive late make the others' waits run out (none where all are late, or none is): every such
+    warp counts, also where warp 0's own wait succeeds. The next call reports it and clears it, and the handle then
+    steps as a fresh one."""
+    lib = _lib.load()
+    mesh, cfg = configs.manufactured(6, p=1, dt=5.0)
+    P, Q = Problem(cfg, mesh), Problem(cfg, mesh)
+    gave_up = C.c_uint32(99)
+    _lib.check(lib.dgsw_check_stage_barrier(P._h, late, 64, C.byref(gave_up)))
+    assert gave_up.value == (0 if late in (0, 15) else 15 & ~late)
+    if gave_up.value:
+        with pytest.raises(DgswError, match="barrier wait"):
+            P.step_serial(1)
+        P.preprocessor_serial()
+    P.step_serial(3)
+    Q.step_serial(3)
+    assert np.array_equal(P.get_state(), Q.get_state())
