@@ -133,6 +133,7 @@ struct dgsw_rkdg_s {
     void* geo = nullptr;    // [4][ne_pad] J^-1
     DBuf<int> fmeta;        // [3][ne_pad] face kinds and slots
     void* fw = nullptr;     // [3][ne_pad] half face length over |J|
+    void* sph = nullptr;    // [spherical_rows][ne_pad] spherical correction factors (spherical runs only)
     void* manning = nullptr;  // [ne_pad] g n^2 per element (Manning friction only)
     Forcing forcing;
     DBuf<int2> fface;      // tide / flow forcing records
@@ -261,6 +262,19 @@ TimeArgs time_args(dgsw_rkdg_s* h, int copy) {
     return T;
 }
 
+// the spherical correction's factors (h->sph), once per handle
+template <int P, typename Real>
+cudaError_t form_spherical(dgsw_rkdg_s* h) {
+    const size_t bytes = (size_t)spherical_rows<P>() * h->ne_pad * sizeof(Real);
+    cudaError_t e = cudaMalloc(&h->sph, bytes);
+    if (e != cudaSuccess) return e;
+    h->device_bytes += (int64_t)bytes;
+    const double cos_lat0 = std::cos(h->cfg.sp_lat0_deg * 3.14159265359 / 180.0);  // the reference's PI
+    spherical_kernel<P, Real><<<(unsigned)((h->ne + 127) / 128), 128, 0, h->stream>>>(
+        h->enodes.p, h->xy.p, cos_lat0, h->cfg.sp_R, (int)h->ne, (int)h->ne_pad, (Real*)h->sph);
+    return cudaGetLastError();
+}
+
 // the current step's time data from the host's t and step
 cudaError_t write_step_time(dgsw_rkdg_s* h) {
     TimeArgs T = time_args(h, h->qswap);
@@ -340,8 +354,7 @@ void fill_stage_args(dgsw_rkdg_s* h, int s, StageArgs<Real>& A) {
     A.fn_set = h->cfg.function_set;
     for (int i = 0; i < 16; ++i) A.fn_params[i] = h->cfg.fn_params[i];
     A.spherical = h->cfg.spherical;
-    A.sp_cos_lat0 = std::cos(h->cfg.sp_lat0_deg * 3.14159265359 / 180.0);  // the reference's PI
-    A.sp_R = h->cfg.sp_R;
+    A.sph = (const Real*)h->sph;
     A.friction = h->cfg.bottom_friction;
     A.friction_cf = h->cfg.friction_cf;
     A.manning = (const Real*)h->manning;
@@ -1070,9 +1083,14 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
             if ((e = h->fval.alloc(2 * (size_t)T.nsets * forcing_values(h))) != cudaSuccess) return cleanup_fail("alloc", e);
             h->device_bytes += (int64_t)h->fval.n * 8;
         }
-        // the forcing data's copies above ran on the default stream, which the handle's stream does not wait for
+        // the copies above ran on the default stream, which the handle's stream does not wait for
         if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess || (e = write_step_time(h)) != cudaSuccess)
             return cleanup_fail("clock", e);
+        if (cfg->spherical) {
+            e = h->fp32 ? (cfg->p == 1 ? form_spherical<1, float>(h) : form_spherical<2, float>(h))
+                        : (cfg->p == 1 ? form_spherical<1, double>(h) : form_spherical<2, double>(h));
+            if (e != cudaSuccess) return cleanup_fail("spherical correction", e);
+        }
         if ((e = h->red.alloc(reduction_partials(h->ne))) != cudaSuccess) return cleanup_fail("alloc", e);
         {
             static L2Rule Rh;
@@ -1511,6 +1529,7 @@ int32_t dgsw_rkdg_destroy(dgsw_handle h) {
     if (h->geo) cudaFree(h->geo);
     h->fmeta.release();
     if (h->fw) cudaFree(h->fw);
+    if (h->sph) cudaFree(h->sph);
     if (h->manning) cudaFree(h->manning);
     h->fface.release();
     h->fcon.release();

@@ -264,7 +264,7 @@ struct StageArgs {
     int fn_set;
     double fn_params[16];
     int spherical;
-    double sp_cos_lat0, sp_R;
+    const Real* sph;  // [spherical_rows][ne_pad] spherical correction factors (null without)
     // bottom friction (swe_source.hpp:29-51): DGSW_FRICTION_NONE / CHEZY / MANNING
     int friction;
     double friction_cf;
@@ -820,57 +820,96 @@ __device__ __noinline__ void ghost_face(const StageArgs<Real>* Ap, unsigned char
     });
 }
 
-// the spherical correction at Gauss point gp of face f
+// The spherical correction cos(phi_0) / cos(y / R) at an element's face and volume Gauss points (geometry alone):
+// rows face * NG + gp, then 3 NG + gp, of [ne_pad] values, formed once per handle. In the stage kernel it was a cosine in
+// FP64 per point, and two per face point as both elements of a face evaluate its flux. 8 steps of 131,072 triangles:
+// tidal channel p = 1 FP64 0.71 -> 0.44 ms, FP32 0.43 -> 0.28, p = 2 FP64 2.09 -> 1.41, FP32 0.99 -> 0.63; wet/dry bowl
+// p = 1 FP64 0.76 -> 0.38, FP32 0.39 -> 0.24.
+template <int P>
+constexpr int spherical_rows() {
+    return 3 * MT<P>::NG + MT<P>::NQ;
+}
 template <int P, typename Real>
-__device__ __forceinline__ Real spherical_factor(const StageArgs<Real>& A, int d, int f, int gp) {
-    constexpr int NG = MT<P>::NG;
-    const double ya = A.xy[A.enodes[((f + 1) % 3) * A.ne_pad + d]].y, yb = A.xy[A.enodes[((f + 2) % 3) * A.ne_pad + d]].y;
-    double wa = 0, wb = 0;
-    sfor<0, NG>([&](auto GP) {
-        constexpr int k = decltype(GP)::value;
-        if (gp == k) wa = MT<P>::fpsi((0 * 3 + 1) * NG + k), wb = MT<P>::fpsi((0 * 3 + 2) * NG + k);
+__global__ void __launch_bounds__(128) spherical_kernel(const int* __restrict__ enodes, const double2* __restrict__ xy,
+                                                        double cos_lat0, double R, int ne, int ne_pad,
+                                                        Real* __restrict__ sph) {
+    constexpr int NG = MT<P>::NG, NQ = MT<P>::NQ;
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= ne) return;
+    double y[3];
+    sfor<0, 3>([&](auto V) { y[decltype(V)::value] = xy[enodes[decltype(V)::value * ne_pad + d]].y; });
+    sfor<0, 3>([&](auto F) {
+        constexpr int f = decltype(F)::value;
+        sfor<0, NG>([&](auto G) {
+            constexpr int g = decltype(G)::value;
+            constexpr double wa = MT<P>::fpsi((0 * 3 + 1) * NG + g), wb = MT<P>::fpsi((0 * 3 + 2) * NG + g);
+            sph[(size_t)(f * NG + g) * ne_pad + d] = (Real)(cos_lat0 / cos((y[(f + 1) % 3] * wa + y[(f + 2) % 3] * wb) / R));
+        });
     });
-    return (Real)(A.sp_cos_lat0 / cos((ya * wa + yb * wb) / A.sp_R));
+    sfor<0, NQ>([&](auto Q) {
+        constexpr int q = decltype(Q)::value;
+        constexpr Real p0 = (Real)MT<P>::psi(0 * NQ + q), p1 = (Real)MT<P>::psi(1 * NQ + q), p2 = (Real)MT<P>::psi(2 * NQ + q);
+        sph[(size_t)(3 * NG + q) * ne_pad + d] = (Real)(cos_lat0 / cos((y[0] * p0 + y[1] * p1 + y[2] * p2) / R));
+    });
 }
 
-// The wet/dry fix-ups of an interface (wd_fixup) seen from one of its elements: own and neighbour are put into
-// the interface's in / ex order, and the own side's doubled flux times w comes back (F likewise). Out of line (interfaces with a
-// dry side only).
-template <int P, typename Real>
-__device__ __noinline__ Val3<Real> wd_fixup_own(const StageArgs<Real>* Ap, int d, int f, int gp, bool is_in, bool wo,
-                                                bool wn, Real oz, Real ox, Real oy, Real ob, Real nz, Real nqx, Real nqy,
-                                                Real nb, Real Nx, Real Ny, Real w, Real F0, Real F1, Real F2) {
-    const StageArgs<Real>& A = *Ap;
-    Real sp = Real(1);
-    if (A.spherical) sp = spherical_factor<P, Real>(A, d, f, gp);
-    const Real g = (Real)A.g, half = Real(0.5) / w, nx = Nx / w, ny = Ny / w, w2 = 2 * w;
-    if (is_in) {
-        const Flux2<Real> r = wd_fixup<Real>(g, oz, ox, oy, nz, nqx, nqy, ob, nb, sp, nx, ny, wo, wn, half * F0, half * F1,
-                                             half * F2);
-        return Val3<Real>{w2 * r.i0, w2 * r.i1, w2 * r.i2};
-    }
-    const Flux2<Real> r = wd_fixup<Real>(g, nz, nqx, nqy, oz, ox, oy, nb, ob, sp, -nx, -ny, wn, wo, -half * F0, -half * F1,
-                                         -half * F2);
-    return Val3<Real>{w2 * r.e0, w2 * r.e1, w2 * r.e2};
+// llf_sides with the spherical correction: sp multiplies the x component of the in side's normal flux and of the normal in
+// both sides' wave speeds (llf_flux, the products regrouped as in llf_sides)
+template <bool PK, typename Real>
+__device__ __forceinline__ void llf_sides_spherical(Real g, const Side<Real>& o, const Side<Real>& n, Two<Real> N, Real sp,
+                                                    bool is_in, Real& F0, Two<Real>& F12) {
+    const Real nxs = sp * N.x;
+    const Real W = sqrt(fma_rn(nxs, nxs, mul_rn(N.y, N.y)));
+    const Two<Real> No = {is_in ? nxs : N.x, N.y}, Nn = {is_in ? N.x : nxs, N.y};
+    const Real fo = fma_rn(o.q.x, No.x, mul_rn(o.q.y, No.y)), fn = fma_rn(n.q.x, Nn.x, mul_rn(n.q.y, Nn.y));
+    const Real po = mul_rn(mul_rn(g, o.ze), fma_rn(Real(0.5), o.ze, o.b));
+    const Real pn = mul_rn(mul_rn(g, n.ze), fma_rn(Real(0.5), n.ze, n.b));
+    const Two<Real> go = fma2<PK, Real>(o.q, mul_rn(fo, o.ih), mul2<PK, Real>(No, po));
+    const Two<Real> gn = fma2<PK, Real>(n.q, mul_rn(fn, n.ih), mul2<PK, Real>(Nn, pn));
+    const Real uo = mul_rn(fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)), o.ih), un = mul_rn(fma_rn(n.q.x, N.x, mul_rn(n.q.y, N.y)), n.ih);
+    const Real lam = fmax(fma_rn(o.c, W, fabs(uo)), fma_rn(n.c, W, fabs(un)));
+    F0 = fma_rn(lam, add_rn(o.ze, -n.ze), add_rn(fo, fn));
+    F12 = fma2<PK, Real>(add2<PK, Real>(o.q, Two<Real>{-n.q.x, -n.q.y}), lam, add2<PK, Real>(go, gn));
 }
 
-// the doubled flux times w of an own side towards n where the spherical correction (sp on the interface's in side
-// only) applies; out of line
-template <int P, typename Real>
-__device__ __noinline__ Val3<Real> spherical_flux(const StageArgs<Real>* Ap, int d, int f, int gp, bool is_in, Real oz,
-                                                  Real ox, Real oy, Real ob, Real nz, Real nqx, Real nqy, Real nb,
-                                                  Real Nx, Real Ny, Real w) {
-    const StageArgs<Real>& A = *Ap;
-    const Real sp = spherical_factor<P, Real>(A, d, f, gp);
-    const Real qo[3] = {oz, ox, oy}, qn[3] = {nz, nqx, nqy};
-    const Real nx = Nx / w, ny = Ny / w, w2 = 2 * w;
-    Real F[3];
-    if (is_in) {
-        llf_flux<Real>((Real)A.g, qo, qn, ob, sp, nx, ny, F);
-        return Val3<Real>{F[0] * w2, F[1] * w2, F[2] * w2};
+// A face Gauss point where the spherical correction applies: the doubled flux times w of the own side, wet/dry fix-ups
+// (wd_fixup) as the own side sees them included. In the fix-ups the own side is the in side. Out of line and without
+// calls of its own, so that the kernel's registers are those of a run without the correction and none are saved here
+// (with a call to wd_fixup instead, 20 % of an FP64 stage of 8,192 triangles went into saving them).
+template <int P, bool WD, typename Real>
+__device__ __noinline__ Val3<Real> spherical_point(const StageArgs<Real>* Ap, const unsigned char* tr, int NS, int own,
+                                                   int slot, int gp, Real sp, bool is_in, bool wet, bool wn, Real Nx,
+                                                   Real Ny, Real w) {
+    constexpr bool PK = sizeof(Real) == 4;
+    const Real g = (Real)Ap->g;
+    const Two<Real> N = {Nx, Ny};
+    Side<Real> o = Trace<P, Real>::get(tr, NS, own, gp, g);
+    Side<Real> n = Trace<P, Real>::get(tr, NS, slot, MT<P>::NG - 1 - gp, g);
+    if (WD && sizeof(Real) == 8) {  // a dry side's trace comes without them
+        if (!wet) complete<Real>(o, g);
+        if (!wn) complete<Real>(n, g);
     }
-    llf_flux<Real>((Real)A.g, qn, qo, nb, sp, -nx, -ny, F);
-    return Val3<Real>{-F[0] * w2, -F[1] * w2, -F[2] * w2};
+    Real F0;
+    Two<Real> F12;
+    llf_sides_spherical<PK, Real>(g, o, n, N, sp, is_in, F0, F12);
+    if (WD && wet != wn) {
+        const Real thr = Real(2e-12) * w;
+        if (F0 > thr) {
+            if (!wet) F0 = Real(0), F12 = {Real(0), Real(0)};  // none leaves a dry element
+        } else if (F0 < -thr) {
+            Real g2 = g, F0w;
+            if (!wn) {  // none comes from a dry neighbour: a reflective wall, the neighbour is the own state mirrored
+                const Real a = Real(-2) * fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)) / (w * w);
+                n = o;
+                n.q = fma2<PK, Real>(N, a, o.q);
+            } else {  // into a dry element: gravity-free momentum flux
+                g2 = o.c = n.c = Real(0);
+            }
+            llf_sides_spherical<PK, Real>(g2, o, n, N, sp, true, F0w, F12);
+            if (!wn) F0 = F0w;
+        }
+    }
+    return Val3<Real>{F0, F12.x, F12.y};
 }
 
 // The master tables in constant memory, for the loops that run rolled (uniform indexes); FP32 entries twice,
@@ -1026,8 +1065,9 @@ __device__ __forceinline__ void stage_bar_arrive(unsigned long long* bar) {
                          (unsigned)__cvta_generic_to_shared(bar))
                      : "memory");
 }
-// polls of the bounded wait. All warps of a CTA arrive, so that a wait that runs out means a fault of this code
-constexpr unsigned STAGE_BAR_POLLS = 1u << 24;
+// polls of the bounded wait, about 4 us each: a second. All warps of a CTA arrive, so that a wait that runs out means a
+// fault of this code
+constexpr unsigned STAGE_BAR_POLLS = 1u << 18;
 // false, and recorded in the status by whichever thread it happens to, when the wait runs out: its element's results
 // stay unwritten, whatever the other warps' waits do
 __device__ __forceinline__ bool stage_bar_wait(unsigned long long* bar, DevStatus* status,
@@ -1261,11 +1301,11 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
     Real q[3][ND], b[3];
     Real Ji00 = Real(0), Ji01 = Real(0), Ji10 = Real(0), Ji11 = Real(0);
     double x0 = 0, y0 = 0, x1 = 0, y1 = 0, x2 = 0, y2 = 0;
-    // the vertex coordinates (analytic source, spherical correction). FP64 at p = 2, whose register budget is
+    // the vertex coordinates (analytic source). FP64 at p = 2, whose register budget is
     // tightest, loads them after the traces
     constexpr bool xy_early = sizeof(Real) == 4 || P == 1;
     auto load_xy = [&]() {
-        if (FSRC || A.spherical) {
+        if (FSRC) {
             const int n0 = A.enodes[d], n1 = A.enodes[P_ + d], n2 = A.enodes[2 * P_ + d];
             const double2 p0 = A.xy[n0], p1 = A.xy[n1], p2 = A.xy[n2];
             x0 = p0.x, y0 = p0.y, x1 = p1.x, y1 = p1.y, x2 = p2.x, y2 = p2.y;
@@ -1399,7 +1439,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
             Real X0 = Ji00, X1 = Ji10;
             if (A.spherical) {
                 const int i = gp;
-                const Real sp = (Real)(A.sp_cos_lat0 / cos((y0 * TB.psi[i][0] + y1 * TB.psi[i][1] + y2 * TB.psi[i][2]) / A.sp_R));
+                const Real sp = A.sph[(3 * NG + i) * P_ + d];
                 X0 *= sp, X1 *= sp;
             }
             const Real U0 = X0 * m.x + Ji01 * m.y, U1 = X1 * m.x + Ji11 * m.y;
@@ -1610,7 +1650,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
     };
     // on: a face between wet elements, or a boundary face of one; these run without branches, so that one face's
     // loads overlap another's arithmetic. special: an interface with one dry side, a levee, the spherical correction;
-    // few elements have one, and a rolled loop takes them afterwards.
+    // few elements have one of the first two, and a rolled loop takes them afterwards.
     bool on[3];
     int special = 0;
 #pragma unroll
@@ -1622,7 +1662,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
         on[f] = any && !sp;
         if (sp) special |= 1 << f;
     }
-    if (!WD || on[0] || on[1] || on[2]) {
+    if (!A.spherical && (!WD || on[0] || on[1] || on[2])) {  // with the correction every face is special
         auto face = [&](auto FF) {
             const auto fc = FF;  // IC<f> (unrolled) or an int
             const int f = fc;
@@ -1673,42 +1713,40 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
             const bool wn = swet[slot] != 0;
             const Two<Real> N = scaled_normal<Real>(f, Ji00, Ji01, Ji10, Ji11);
             const Real iw = Real(1) / w, thr = Real(2e-12) * w;
+            Real sp_next = A.spherical ? A.sph[f * NG * P_ + d] : Real(1);  // loaded a point ahead
 #pragma unroll 1
             for (int gp = 0; gp < NG; ++gp) {
-                Side<Real> o = TR::get(tr, NS, 3 * tid + f, gp, g);
-                Side<Real> n = TR::get(tr, NS, slot, NG - 1 - gp, g);
-                if (WD && sizeof(Real) == 8) {  // a dry side's trace comes without them
-                    if (!wet) complete<Real>(o, g);
-                    if (!wn) complete<Real>(n, g);
-                }
                 Real F0;
                 Two<Real> F12;
                 if (A.spherical) {
-                    Val3<Real> r = spherical_flux<P, Real>(&A, d, f, gp, is_in, o.ze, o.q.x, o.q.y, o.b, n.ze, n.q.x, n.q.y,
-                                                           n.b, N.x, N.y, w);
-                    if (WD && wet != wn)
-                        r = wd_fixup_own<P, Real>(&A, d, f, gp, is_in, wet, wn, o.ze, o.q.x, o.q.y, o.b, n.ze, n.q.x, n.q.y,
-                                                  n.b, N.x, N.y, w, r.v0, r.v1, r.v2);
+                    const Real sp = sp_next;
+                    if (gp + 1 < NG) sp_next = A.sph[(f * NG + gp + 1) * P_ + d];
+                    const Val3<Real> r = spherical_point<P, WD, Real>(&A, tr, NS, 3 * tid + f, slot, gp, sp, is_in, wet, wn,
+                                                                      N.x, N.y, w);
                     F0 = r.v0, F12 = {r.v1, r.v2};
                 } else {
+                    Side<Real> o = TR::get(tr, NS, 3 * tid + f, gp, g);
+                    Side<Real> n = TR::get(tr, NS, slot, NG - 1 - gp, g);
+                    if (WD && sizeof(Real) == 8) {  // a dry side's trace comes without them
+                        if (!wet) complete<Real>(o, g);
+                        if (!wn) complete<Real>(n, g);
+                    }
                     llf_sides<PK, Real>(g, o, n, N, w, F0, F12);
-                    if (WD && wet != wn) {
-                        // the fix-ups of wd_fixup (rkdg_swe_is_internal.hpp:47-90) as the own side sees them
-                        if (F0 > thr) {
-                            if (!wet) F0 = Real(0), F12 = {Real(0), Real(0)};  // none leaves a dry element
-                        } else if (F0 < -thr) {
-                            if (!wn) {  // none comes from a dry neighbour: a reflective wall
-                                // the mirrored state's flux in closed form: no mass through the wall, and twice the
-                                // pressure and the normal momentum's upwinding on it
-                                const Real fo = fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)), uo = fo * o.ih;
-                                const Real a = (uo + fabs(uo) + o.c * w) * (2 * fo * iw * iw) +
-                                               2 * (g * o.ze * (Real(0.5) * o.ze + o.b));
-                                F0 = Real(0), F12 = {a * N.x, a * N.y};
-                            } else {  // into a dry element: gravity-free momentum flux
-                                o.c = n.c = Real(0);
-                                Real F0g;
-                                llf_sides<PK, Real>(Real(0), o, n, N, w, F0g, F12);
-                            }
+                    // the fix-ups of wd_fixup (rkdg_swe_is_internal.hpp:47-90) as the own side sees them
+                    if (F0 > thr) {
+                        if (!wet) F0 = Real(0), F12 = {Real(0), Real(0)};  // none leaves a dry element
+                    } else if (F0 < -thr) {
+                        if (!wn) {  // none comes from a dry neighbour: a reflective wall
+                            // the mirrored state's flux in closed form: no mass through the wall, and twice the
+                            // pressure and the normal momentum's upwinding on it
+                            const Real fo = fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)), uo = fo * o.ih;
+                            const Real a = (uo + fabs(uo) + o.c * w) * (2 * fo * iw * iw) +
+                                           2 * (g * o.ze * (Real(0.5) * o.ze + o.b));
+                            F0 = Real(0), F12 = {a * N.x, a * N.y};
+                        } else {  // into a dry element: gravity-free momentum flux
+                            o.c = n.c = Real(0);
+                            Real F0g;
+                            llf_sides<PK, Real>(Real(0), o, n, N, w, F0g, F12);
                         }
                     }
                 }

@@ -333,7 +333,7 @@ int32_t dgsw_check_internal_flux(int32_t precision, int64_t n, double g, const d
 int32_t dgsw_check_wetting_drying(int64_t n, const double* q, const double* bath_vrtx, double h_o,
                                   const uint8_t* wet_in, double* q_out, uint8_t* wet_out, uint8_t* went_dry);
 /* the stage kernel's bounded barrier wait, on a handle: one CTA of four warps of which those in `late_warps`
- * (bit per warp) arrive only when the others' waits have ended, so that these run out after `polls` (1 to 2^24)
+ * (bit per warp) arrive only when the others' waits have ended, so that these run out after `polls` (1 to 2^18)
  * polls. gave_up gets a bit per warp whose wait ran out; they are recorded in the handle as a stage's are, and its
  * next stage or step call returns DGSW_ERR_CUDA once. */
 int32_t dgsw_check_stage_barrier(dgsw_handle h, uint32_t late_warps, uint32_t polls, uint32_t* gave_up);

@@ -558,6 +558,55 @@ def test_spherical_correction_with_forcing_and_levees(oracle, which):
     assert e <= 1e-12, e
 
 
+def _north(mesh, cfg):
+    """The problem moved to about 30 degrees north on the projection cylinder."""
+    mesh.node_xyz = mesh.node_xyz.copy()
+    mesh.node_xyz[:, 1] += 3.3e6
+    cfg.spherical = True
+    cfg.sp_lat0_deg = 30.0
+    return mesh, cfg
+
+
+@pytest.mark.parametrize("precision,bar", [("fp64", 1e-9), ("fp32", 1e-4)])
+@pytest.mark.parametrize("p,tile", [(1, 128), (1, 256), (2, 128)])
+def test_spherical_correction_at_a_shoreline(oracle, p, tile, precision, bar):
+    """The spherical correction together with wetting/drying: a bowl with a hump that floods and drains its shore, with
+    wet in sides against dry ex sides and the other way round. FP64 as for the other wet/dry runs; FP32: the
+    pressure and bathymetry terms, g h^2 / 2 with h up to 10 m, cancel to a surface slope's worth, which leaves
+    2^-24 x 10 x (10 / 0.5 m) of the momentum's scale, 1e-5, per unit of condition; the bar is ten times that."""
+    mesh, cfg = configs.bowl_humps(nq=40, dt=1.0, limiter=False, precision=precision)
+    mesh, cfg = _north(mesh, cfg)
+    cfg.p, cfg.rk_nstages, cfg.rk_order = p, p + 1, p + 1
+    cfg.fn_params = configs.humps_params([(3.0, 500.0, 3.3e6 + 2300.0, 600.0)])
+    P = Problem(cfg, mesh, tile=tile)
+    O = oracle.problem(cfg, mesh, n_threads=8)
+    intf = P.topology()[2]
+    before = P.get_wet().astype(bool)
+    in_wet, ex_wet = before[intf[:, 0]], before[intf[:, 1]]
+    assert (in_wet & ~ex_wet).sum() > 20 and (~in_wet & ex_wet).sum() > 20
+    P.step_serial(160)
+    O.step(160)
+    wg, wo = P.get_wet(), O.get_wet()
+    assert (wo.astype(bool) != before).sum() > 20  # the shoreline has moved
+    assert np.count_nonzero(wg != wo) <= (0 if precision == "fp64" else 2)
+    e = rel_err(P.get_state(), O.get_state())
+    assert e <= bar, e
+
+
+def test_spherical_correction_fp32(oracle):
+    """FP32 arithmetic with the spherical correction on the forced channel, without and with stage increments: the
+    bar of the FP32 channel without it."""
+    mesh, cfg64 = _north(*configs.tidal_channel(p=2, rk=(3, 3), dt=1.0))
+    cfg = _north(*configs.tidal_channel(p=2, rk=(3, 3), dt=1.0, precision="fp32"))[1]
+    O = oracle.problem(cfg64, mesh, n_threads=8)
+    O.step(300)
+    for fp64_stages in (False, True):
+        P = Problem(cfg, mesh, fp64_stages=fp64_stages)
+        P.step_serial(300)
+        e = rel_err(P.get_state(), O.get_state())
+        assert e < 1e-4, e
+
+
 def test_manning_friction_in_drying_cells(oracle):
     """Manning friction while the levee floods dry land (depths near h_o make g n^2 / h^(1/3) large):
     wet counts within 0.5 %, state within 1e-9."""
