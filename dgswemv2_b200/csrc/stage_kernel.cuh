@@ -986,13 +986,14 @@ struct Smem {
     static __host__ __device__ size_t off_wet(int tile, int mh) {
         return (size_t)16 * MT<P>::NG * Trace<P, Real>::NV * nslot(tile, mh);
     }
-    // halo staging: the state and bathymetry modes of each halo face's element, copied asynchronously
+    // halo staging (FP32): the state and bathymetry modes of each halo face's element, copied asynchronously
+    static constexpr bool staged = sizeof(Real) == 4;
     static __host__ __device__ size_t off_halo(int tile, int mh) { return off_wet(tile, mh) + al((size_t)nslot(tile, mh)); }
     static __host__ __device__ size_t off_hbath(int tile, int mh) {
         return off_halo(tile, mh) + al(sizeof(double) * (size_t)3 * ND * mh);
     }
     static __host__ __device__ size_t bytes(int tile, int mh) {
-        return off_hbath(tile, mh) + al(sizeof(Real) * (size_t)3 * mh);
+        return staged ? off_hbath(tile, mh) + al(sizeof(Real) * (size_t)3 * mh) : off_halo(tile, mh);
     }
 };
 
@@ -1222,8 +1223,15 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
         }
     };
     bool wet = false;
-    // with capped tiles (at most TILE / 2 halo and boundary faces) thread h < nh owns halo face h: its record is
-    // loaded now and its element's data copied asynchronously into shared memory while the own traces are formed
+    // FP32 with capped tiles (at most TILE / 2 halo and boundary faces): thread h < nh owns halo face h, its record is
+    // loaded now and its element's data copied asynchronously into shared memory while the own traces are formed.
+    // FP64 loads the halo elements after its own traces, in every tile: the staging area, 6 KB (p = 1) or 11 KB (p = 2) a
+    // CTA, put the resident CTAs' shared memory above 196 KB, which leaves the L1 28 KB for 512 or 384 threads' loads in
+    // flight instead of 60. Measured per 8 steps of 524,288 triangles, with staging -> without: p = 1 closed basin 1.17 ->
+    // 0.84 ms, channel 1.25 -> 0.96, bowl 1.03 -> 1.02; p = 2 closed basin 3.29 -> 2.68 ms, channel 3.60 -> 2.95,
+    // manufactured 4.15 -> 3.54, bowl 2.91 -> 2.43. (Staged in the halo face's own trace slot, which takes no memory, p = 1
+    // 0.92 ms; tiles sized to the mesh run 10 to 15 % slower with copies than with loads.)
+    constexpr bool ASYNC = CAPPED && SM::staged;
     const int4 ti = A.tiles[tile];
     const int hoff = ti.x, nh = ti.y;
     // FP64: one thread asks L2 for the rows this CTA reads only at its end, the RK combination's earlier
@@ -1253,7 +1261,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
         }
     }
     int2 hrec = make_int2(0, -1);
-    if (CAPPED && tid < nh) hrec = A.halo[hoff + tid];
+    if (ASYNC && tid < nh) hrec = A.halo[hoff + tid];
     bool hwet = false;
     // stage increments: the halo staging holds q0f in its first 3 ND Real rows and d_s in the next 3 ND
     // (the same bytes as 3 ND doubles)
@@ -1317,7 +1325,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
     Real fw[3];
     if (active) {
         load_state(q, d);
-        if (CAPPED && hrec.y >= 0) issue_halo_copies();
+        if (ASYNC && hrec.y >= 0) issue_halo_copies();
 #pragma unroll
         for (int k = 0; k < 3; ++k) b[k] = A.bath[k * P_ + d];
         wet = A.wet_in[d] != 0;
@@ -1363,7 +1371,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
         }
         swet[slot] = w ? 1 : 0;
     };
-    if (CAPPED) {
+    if (ASYNC) {
         if (hrec.y >= 0) {
             if (!active) issue_halo_copies();  // threads past the last element of the last tile
             const int h = tid;
@@ -1901,8 +1909,8 @@ cudaError_t launch_stage_impl(const StageArgs<Real>& A, int ntiles, int max_halo
     const bool capped = allow_capped && max_halo <= TileCap<TILE>::halo;
     auto kern = capped ? rkdg_stage_kernel<P, Real, WD, FSRC, FRIC, TILE, true, OCC, SPLIT>
                        : rkdg_stage_kernel<P, Real, WD, FSRC, FRIC, TILE, false, OCC, SPLIT>;
-    // the run-time-stride kernel loads its halo faces' elements straight from global memory and never
-    // touches the halo staging area (every use of it is under CAPPED), so its allocation ends there
+    // the run-time-stride kernel loads its halo faces' elements straight from global memory, so its allocation ends
+    // before the staging area
     const size_t smem = capped ? Smem<P, Real>::bytes(TILE, TileCap<TILE>::halo) : Smem<P, Real>::off_halo(TILE, max_halo);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
