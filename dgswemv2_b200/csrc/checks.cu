@@ -1,5 +1,5 @@
-// Kernel self-checks: the stage kernel's own device functions (llf_flux, the ISP::Internal wet/dry
-// fix-ups, wetting_drying from stage_kernel.cuh) run by small kernels on caller data, so that the
+// Kernel self-checks: the stage kernel's own device functions (llf_sides and llf_sides_spherical, the wet/dry fix-ups
+// wd_fixup and wd_fixup_spherical, wetting_drying from stage_kernel.cuh) run by small kernels on caller data, so that the
 // reference's known-answer vectors (test/test_llf_flux.cpp, test/test_wetting_drying.cpp) and the oracle
 // can be checked against the CUDA code itself rather than only through whole runs.
 // Host arrays in and out; device buffers are allocated per call (these are test entry points).
@@ -18,10 +18,39 @@ int set_last_error(int code, const std::string& msg);
 
 namespace {
 
-using dgsw::Flux2;
+// One side's flux at a Gauss point as the face loop forms it: o towards n along the unit normal (nx, ny) scaled by w. The LLF
+// flux takes the bathymetry b on both sides, the wet/dry fix-ups the own side's, as the reference does; on a mesh they
+// are the same values.
+template <typename Real>
+__device__ void side_flux(Real g, const Real qo[3], const Real qn[3], Real b, Real b_own, Real sp, Real nx, Real ny, Real w,
+                          bool is_in, bool fix, bool wet, bool wn, Real F[3]) {
+    constexpr bool PK = sizeof(Real) == 4;
+    dgsw::Side<Real> o, n;
+    o.q = {qo[1], qo[2]}, o.ze = qo[0], o.b = b;
+    n.q = {qn[1], qn[2]}, n.ze = qn[0], n.b = b;
+    dgsw::complete<Real>(o, g);
+    dgsw::complete<Real>(n, g);
+    const dgsw::Two<Real> N = {w * nx, w * ny};
+    dgsw::Two<Real> F12;
+    if (sp == Real(1))
+        dgsw::llf_sides<PK, Real>(g, o, n, N, w, F[0], F12);
+    else
+        dgsw::llf_sides_spherical<PK, Real>(g, o, n, N, sp, is_in, F[0], F12);
+    if (fix && !(wet && wn)) {
+        o.b = n.b = b_own;
+        dgsw::complete<Real>(o, g);
+        dgsw::complete<Real>(n, g);
+        if (sp == Real(1))
+            dgsw::wd_fixup<PK, Real>(g, o, n, N, w, wet, wn, F[0], F12);
+        else
+            dgsw::wd_fixup_spherical<PK, Real>(g, o, n, N, w, sp, wet, wn, F[0], F12);
+    }
+    const Real half = Real(0.5) / w;
+    F[0] *= half, F[1] = half * F12.x, F[2] = half * F12.y;
+}
 
-// the interface Gauss point of the stage kernel's face loop: LLF (llf_sides, or llf_flux where sp differs from 1) with sp on the in
-// side, F_ex = -F_in, and the wet/dry fix-ups when either side is dry (rkdg_swe_is_internal.hpp:26-95)
+// the interface Gauss point as its two elements see it, each with its own weight: LLF with sp on the in side, and the
+// wet/dry fix-ups where one side is dry (rkdg_swe_is_internal.hpp:26-95)
 template <typename Real>
 __global__ void check_flux_kernel(int n, Real g, const double* __restrict__ qin, const double* __restrict__ qex,
                                   const double* __restrict__ bin, const double* __restrict__ bex,
@@ -33,34 +62,15 @@ __global__ void check_flux_kernel(int n, Real g, const double* __restrict__ qin,
     const Real qi[3] = {(Real)qin[3 * i], (Real)qin[3 * i + 1], (Real)qin[3 * i + 2]};
     const Real qe[3] = {(Real)qex[3 * i], (Real)qex[3 * i + 1], (Real)qex[3 * i + 2]};
     const Real nx = (Real)nrm[2 * i], ny = (Real)nrm[2 * i + 1];
+    const bool wa = !internal || wet_in[i] != 0, wb = !internal || wet_ex[i] != 0;
     Real F[3];
-    if ((Real)sp[i] == Real(1)) {
-        // the face loop's form: both sides on the in side's bathymetry, a unit normal, the doubled flux
-        dgsw::Side<Real> a, b;
-        a.q = {qi[1], qi[2]}, a.ze = qi[0], a.b = (Real)bin[i];
-        b.q = {qe[1], qe[2]}, b.ze = qe[0], b.b = (Real)bin[i];
-        dgsw::complete<Real>(a, g);
-        dgsw::complete<Real>(b, g);
-        dgsw::Two<Real> F12;
-        dgsw::llf_sides<sizeof(Real) == 4, Real>(g, a, b, dgsw::Two<Real>{nx, ny}, Real(1), F[0], F12);
-        F[0] *= Real(0.5), F[1] = Real(0.5) * F12.x, F[2] = Real(0.5) * F12.y;
-    } else {
-        dgsw::llf_flux<Real>(g, qi, qe, (Real)bin[i], (Real)sp[i], nx, ny, F);
-    }
-    Real E[3] = {-F[0], -F[1], -F[2]};
-    if (internal) {
-        const bool wa = wet_in[i] != 0, wb = wet_ex[i] != 0;
-        if (!(wa && wb)) {
-            const Flux2<Real> r = dgsw::wd_fixup<Real>(g, qi[0], qi[1], qi[2], qe[0], qe[1], qe[2], (Real)bin[i],
-                                                       (Real)bex[i], (Real)sp[i], nx, ny, wa, wb, F[0], F[1], F[2]);
-            F[0] = r.i0, F[1] = r.i1, F[2] = r.i2;
-            E[0] = r.e0, E[1] = r.e1, E[2] = r.e2;
-        }
-    }
-    for (int v = 0; v < 3; ++v) {
-        Fin[3 * i + v] = (double)F[v];
-        if (Fex) Fex[3 * i + v] = (double)E[v];
-    }
+    side_flux<Real>(g, qi, qe, (Real)bin[i], (Real)bin[i], (Real)sp[i], nx, ny, Real(0.3) * (1 + i % 7), true, internal, wa, wb,
+                    F);
+    for (int v = 0; v < 3; ++v) Fin[3 * i + v] = (double)F[v];
+    if (!Fex) return;
+    side_flux<Real>(g, qe, qi, (Real)bin[i], internal ? (Real)bex[i] : (Real)bin[i], (Real)sp[i], -nx, -ny,
+                    Real(0.17) * (1 + i % 5), false, internal, wb, wa, F);
+    for (int v = 0; v < 3; ++v) Fex[3 * i + v] = (double)F[v];
 }
 
 // the stage kernel's wetting/drying pass (FP64 in both precisions) on p = 1 modal states

@@ -366,53 +366,30 @@ __device__ __forceinline__ Two<Real> scaled_normal(int f, Real Ji00, Real Ji01, 
     return {-Ji10, -Ji11};
 }
 
-// land boundary ghost state (normal momentum mirrored) + LLF, rkdg_swe_bc_land.hpp:68-86
-template <typename Real>
-__device__ __forceinline__ void land_flux(Real g, Real nx, Real ny, const Real qin[3], Real bath, Real sp, Real F[3]) {
-    const Real tx = -ny, ty = nx;
-    const Real qn_ex = -(qin[1] * nx + qin[2] * ny);
-    const Real qt_ex = qin[1] * tx + qin[2] * ty;
-    Real qex[3];
-    qex[0] = qin[0];
-    qex[1] = qn_ex * nx + qt_ex * tx;
-    qex[2] = qn_ex * ny + qt_ex * ty;
-    llf_flux<Real>(g, qin, qex, bath, sp, nx, ny, F);
-}
-
-// both sides' fluxes of an interface Gauss point, returned by value from wd_fixup
-template <typename Real>
-struct Flux2 {
-    Real i0, i1, i2, e0, e1, e2;
-};
-
-// Wet/dry fix-ups of ISP::Internal (rkdg_swe_is_internal.hpp:47-90) for an interface whose LLF
-// ze-flux exceeds 1e-12 in magnitude with one side dry; the ex-side flux starts as -F. Out of line
-// (taken on few edges only), with its arguments and results passed by value so that the call site
-// keeps them in registers.
-template <typename Real>
-__device__ __noinline__ Flux2<Real> wd_fixup(Real g, Real qi0, Real qi1, Real qi2, Real qe0, Real qe1, Real qe2,
-                                             Real bi, Real be, Real sp, Real nx, Real ny, bool wa, bool wb, Real F0,
-                                             Real F1, Real F2) {
-    const Real qi[3] = {qi0, qi1, qi2}, qe[3] = {qe0, qe1, qe2};
-    Real Fi[3] = {F0, F1, F2}, Fe[3] = {-F0, -F1, -F2};
-    if (Fi[0] > Real(1e-12)) {
-        if (!wa) {  // water flowing from the dry in-side: zero flux there, reflective wall on the ex side
-            Fi[0] = Fi[1] = Fi[2] = Real(0);
-            land_flux<Real>(g, -nx, -ny, qe, be, sp, Fe);
-        } else if (!wb) {  // water flowing into the dry ex-side: gravity-free LLF there
-            llf_flux<Real>(Real(0), qe, qi, be, sp, -nx, -ny, Fe);
-            Fe[0] = -Fi[0];
-        }
-    } else if (Fi[0] < Real(-1e-12)) {
-        if (!wb) {
-            Fe[0] = Fe[1] = Fe[2] = Real(0);
-            land_flux<Real>(g, nx, ny, qi, bi, sp, Fi);
-        } else if (!wa) {
-            llf_flux<Real>(Real(0), qi, qe, bi, sp, nx, ny, Fi);
-            Fi[0] = -Fe[0];
+// Wet/dry fix-ups of ISP::Internal (rkdg_swe_is_internal.hpp:47-90) for an interface with one dry side whose LLF
+// ze-flux exceeds 1e-12 in magnitude, as the own side sees them: F0, F12 is its flux towards n (llf_sides: doubled,
+// times w) before and after. The reference's two branches by the flux's sign are one here, since a side's flux is
+// negative where the other's is positive: water leaves a dry element (none does), or comes from a dry neighbour (none
+// does, a reflective wall), or flows into a dry element (without gravity).
+template <bool PK, typename Real>
+__device__ __forceinline__ void wd_fixup(Real g, Side<Real> o, Side<Real> n, Two<Real> N, Real w, bool wet, bool wn, Real& F0,
+                                         Two<Real>& F12) {
+    const Real iw = Real(1) / w, thr = Real(2e-12) * w;
+    if (F0 > thr) {
+        if (!wet) F0 = Real(0), F12 = {Real(0), Real(0)};
+    } else if (F0 < -thr) {
+        if (!wn) {
+            // the mirrored state's flux (rkdg_swe_bc_land.hpp:68-86) in closed form: no mass through the wall, and twice
+            // the pressure and the normal momentum's upwinding on it
+            const Real fo = fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)), uo = fo * o.ih;
+            const Real a = (uo + fabs(uo) + o.c * w) * (2 * fo * iw * iw) + 2 * (g * o.ze * (Real(0.5) * o.ze + o.b));
+            F0 = Real(0), F12 = {a * N.x, a * N.y};
+        } else {
+            o.c = n.c = Real(0);
+            Real F0g;
+            llf_sides<PK, Real>(Real(0), o, n, N, w, F0g, F12);
         }
     }
-    return Flux2<Real>{Fi[0], Fi[1], Fi[2], Fe[0], Fe[1], Fe[2]};
 }
 
 // three values returned by value from the out-of-line helpers below: an output array passed by
@@ -875,10 +852,31 @@ __device__ __forceinline__ void llf_sides_spherical(Real g, const Side<Real>& o,
     F12 = fma2<PK, Real>(add2<PK, Real>(o.q, Two<Real>{-n.q.x, -n.q.y}), lam, add2<PK, Real>(go, gn));
 }
 
+// wd_fixup with the spherical correction: the own side is the in side of the wall's and of the gravity-free flux, and the
+// wall's mass flux, whose two halves no longer cancel, stays (as in the reference)
+template <bool PK, typename Real>
+__device__ __forceinline__ void wd_fixup_spherical(Real g, Side<Real> o, Side<Real> n, Two<Real> N, Real w, Real sp, bool wet,
+                                                   bool wn, Real& F0, Two<Real>& F12) {
+    const Real thr = Real(2e-12) * w;
+    if (F0 > thr) {
+        if (!wet) F0 = Real(0), F12 = {Real(0), Real(0)};
+    } else if (F0 < -thr) {
+        Real Fw;
+        if (!wn) {  // the neighbour is the own state mirrored
+            const Real a = Real(-2) * fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)) / (w * w);
+            n = o;
+            n.q = fma2<PK, Real>(N, a, o.q);
+        } else {
+            g = o.c = n.c = Real(0);
+        }
+        llf_sides_spherical<PK, Real>(g, o, n, N, sp, true, Fw, F12);
+        if (!wn) F0 = Fw;
+    }
+}
+
 // A face Gauss point where the spherical correction applies: the doubled flux times w of the own side, wet/dry fix-ups
-// (wd_fixup) as the own side sees them included. In the fix-ups the own side is the in side. Out of line and without
-// calls of its own, so that the kernel's registers are those of a run without the correction and none are saved here
-// (with a call to wd_fixup instead, 20 % of an FP64 stage of 8,192 triangles went into saving them).
+// included. Out of line and without calls of its own, so that the kernel's registers are those of a run without the
+// correction and none are saved here (with a call inside, 20 % of an FP64 stage of 8,192 triangles went into saving them).
 template <int P, bool WD, typename Real>
 __device__ __noinline__ Val3<Real> spherical_point(const StageArgs<Real>* Ap, const unsigned char* tr, int NS, int own,
                                                    int slot, int gp, Real sp, bool is_in, bool wet, bool wn, Real Nx,
@@ -895,23 +893,7 @@ __device__ __noinline__ Val3<Real> spherical_point(const StageArgs<Real>* Ap, co
     Real F0;
     Two<Real> F12;
     llf_sides_spherical<PK, Real>(g, o, n, N, sp, is_in, F0, F12);
-    if (WD && wet != wn) {
-        const Real thr = Real(2e-12) * w;
-        if (F0 > thr) {
-            if (!wet) F0 = Real(0), F12 = {Real(0), Real(0)};  // none leaves a dry element
-        } else if (F0 < -thr) {
-            Real g2 = g, F0w;
-            if (!wn) {  // none comes from a dry neighbour: a reflective wall, the neighbour is the own state mirrored
-                const Real a = Real(-2) * fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)) / (w * w);
-                n = o;
-                n.q = fma2<PK, Real>(N, a, o.q);
-            } else {  // into a dry element: gravity-free momentum flux
-                g2 = o.c = n.c = Real(0);
-            }
-            llf_sides_spherical<PK, Real>(g2, o, n, N, sp, true, F0w, F12);
-            if (!wn) F0 = F0w;
-        }
-    }
+    if (WD && wet != wn) wd_fixup_spherical<PK, Real>(g, o, n, N, w, sp, wet, wn, F0, F12);
     return Val3<Real>{F0, F12.x, F12.y};
 }
 
@@ -1743,7 +1725,6 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
             const int slot = fm >> 4;
             const bool wn = swet[slot] != 0;
             const Two<Real> N = scaled_normal<Real>(f, Ji00, Ji01, Ji10, Ji11);
-            const Real iw = Real(1) / w, thr = Real(2e-12) * w;
             Real sp_next = A.spherical ? A.sph[f * NG * P_ + d] : Real(1);  // loaded a point ahead
 #pragma unroll 1
             for (int gp = 0; gp < NG; ++gp) {
@@ -1763,23 +1744,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
                         if (!wn) complete<Real>(n, g);
                     }
                     llf_sides<PK, Real>(g, o, n, N, w, F0, F12);
-                    // the fix-ups of wd_fixup (rkdg_swe_is_internal.hpp:47-90) as the own side sees them
-                    if (F0 > thr) {
-                        if (!wet) F0 = Real(0), F12 = {Real(0), Real(0)};  // none leaves a dry element
-                    } else if (F0 < -thr) {
-                        if (!wn) {  // none comes from a dry neighbour: a reflective wall
-                            // the mirrored state's flux in closed form: no mass through the wall, and twice the
-                            // pressure and the normal momentum's upwinding on it
-                            const Real fo = fma_rn(o.q.x, N.x, mul_rn(o.q.y, N.y)), uo = fo * o.ih;
-                            const Real a = (uo + fabs(uo) + o.c * w) * (2 * fo * iw * iw) +
-                                           2 * (g * o.ze * (Real(0.5) * o.ze + o.b));
-                            F0 = Real(0), F12 = {a * N.x, a * N.y};
-                        } else {  // into a dry element: gravity-free momentum flux
-                            o.c = n.c = Real(0);
-                            Real F0g;
-                            llf_sides<PK, Real>(Real(0), o, n, N, w, F0g, F12);
-                        }
-                    }
+                    wd_fixup<PK, Real>(g, o, n, N, w, wet, wn, F0, F12);
                 }
                 const Real wg = Real(-0.5) * TB.gw[gp];
                 lift(f, gp, F0 * wg, mul2<PK, Real>(F12, wg));

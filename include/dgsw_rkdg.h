@@ -323,7 +323,8 @@ int32_t dgsw_mlp_adam(float* d_params, float* d_m, float* d_v, const float* d_gr
 int32_t dgsw_check_llf_flux(int32_t precision, int64_t n, double g, const double* q_in, const double* q_ex,
                             const double* bath, const double* sp, const double* normal, double* F);
 /* ISP::Internal::ComputeFlux at one Gauss point (rkdg_swe_is_internal.hpp:26-95): LLF, F_ex = -F_in, and
- * the wet/dry fix-ups for a dry side (wet flags [n] of each side, bathymetry of each side) */
+ * the wet/dry fix-ups for a dry side (wet flags [n] of each side, bathymetry of each side). Formed as the stage
+ * kernel does, once from each side, each along its own scaled normal. */
 int32_t dgsw_check_internal_flux(int32_t precision, int64_t n, double g, const double* q_in, const double* q_ex,
                                  const double* bath_in, const double* bath_ex, const double* sp, const double* normal,
                                  const uint8_t* wet_in, const uint8_t* wet_ex, double* F_in, double* F_ex);

@@ -1,5 +1,5 @@
 """The reference's known-answer vectors through the CUDA device code itself (the library's kernel
-self-check entry points run the stage kernel's llf_flux, ISP::Internal fix-ups and wetting_drying):
+self-check entry points run the stage kernel's flux, ISP::Internal fix-ups and wetting_drying):
 
 - LLF: the three configurations of test/test_llf_flux.cpp:66-171 (tests/golden/llf_flux.json), FP64 within
   the reference's own tolerance (100 eps relative), FP32 within 2e-6 relative;
@@ -136,6 +136,48 @@ def test_internal_flux_with_wet_dry_fixups_against_the_oracle(oracle):
             kinds.add((int(wet_in[k]), int(wet_ex[k]), bool(F[0] > 0)))
     # every branch of the fix-up ran
     assert len(kinds) >= 6, kinds
+
+
+@pytest.mark.parametrize("precision,eps", [(_lib.DGSW_FP64, 2.0**-53), (_lib.DGSW_FP32, 2.0**-24)])
+@pytest.mark.parametrize("spherical", [False, True])
+def test_internal_flux_from_both_sides_and_about_the_threshold(oracle, precision, eps, spherical):
+    """The flux and its fix-ups as each element forms them, with the bathymetry continuous across the face as on a mesh:
+    every wet/dry combination, mass fluxes of either sign on both sides of the 1e-12 threshold, without and with the
+    spherical factor, against the oracle. Bar: 100 roundings of the largest term that enters, g h^2 with h <= 4 m and
+    |q|^2 / h; about the threshold, where surface and bathymetry terms cancel in the mass flux exactly (equal depths) or
+    to a rounding of the flux itself, 1e-4 of it."""
+    rng = np.random.default_rng(12)
+    n, g = 4096, 9.81
+    f32 = lambda a: np.float32(a).astype(np.float64)  # the same inputs in both precisions
+    bath = f32(rng.uniform(0.5, 3.0, n))
+    qi = f32(np.stack([rng.uniform(-0.3, 0.5, n), rng.normal(0, 0.5, n), rng.normal(0, 0.5, n)], 1))
+    qe = f32(np.stack([rng.uniform(-0.3, 0.5, n), rng.normal(0, 0.5, n), rng.normal(0, 0.5, n)], 1))
+    th = rng.uniform(0, 2 * np.pi, n)
+    # unit to FP64's rounding: the kernel's wave speed takes |n| = 1, so rounding n to FP32 here would move the flux by
+    # 2^-24 (|u| + c) |dq|, up to 6e-8 x 8 x 3, against the oracle's, which forms |n|
+    nrm = np.stack([np.cos(th), np.sin(th)], 1)
+    sp = f32(rng.uniform(0.8, 1.25, n)) if spherical else np.ones(n)
+    small = np.arange(n) >= n // 2  # both sides the same state, its normal momentum about the threshold
+    qi[small, 1:] = f32(rng.choice([-3.0, -0.7, -0.3, 0.3, 0.7, 3.0], small.sum())[:, None] * 1e-12 * nrm[small])
+    qe[small] = qi[small]
+    wet = rng.integers(0, 4, n)
+    wet_in, wet_ex = (wet & 1).astype(np.uint8), (wet >> 1).astype(np.uint8)
+    Fi, Fe = np.zeros((n, 3)), np.zeros((n, 3))
+    lib = _lib.load()
+    _lib.check(lib.dgsw_check_internal_flux(precision, n, g, dp(qi), dp(qe), dp(bath), dp(bath), dp(sp), dp(nrm),
+                                            up(wet_in), up(wet_ex), dp(Fi), dp(Fe)))
+    kinds = set()
+    for k in range(n):
+        ri, re_ = oracle.internal_flux(g, qi[k], qe[k], bath[k], bath[k], sp[k], nrm[k], wet_in[k], wet_ex[k])
+        h = bath[k] + np.array([qi[k, 0], qe[k, 0]])
+        scale = g * 16.0 + max((qi[k, 1:] ** 2).sum() / h[0], (qe[k, 1:] ** 2).sum() / h[1])
+        assert np.abs(Fi[k] - ri).max() <= 100 * eps * scale, (k, Fi[k], ri)
+        assert np.abs(Fe[k] - re_).max() <= 100 * eps * scale, (k, Fe[k], re_)
+        if small[k]:
+            assert abs(Fi[k, 0] - ri[0]) <= 1e-16 and abs(Fe[k, 0] - re_[0]) <= 1e-16, (k, Fi[k], ri, Fe[k], re_)
+        F = oracle.llf_flux(g, qi[k], qe[k], bath[k], sp[k], nrm[k])
+        kinds.add((int(wet[k]), bool(small[k]), int(np.sign(F[0])) * int(abs(F[0]) > 1e-12)))
+    assert len(kinds) >= 4 * 2 + 4 * 3, sorted(kinds)  # every combination and sign, and below the threshold
 
 
 @pytest.mark.parametrize("late", [0, 1, 2, 8, 5, 15])
