@@ -146,7 +146,7 @@ struct dgsw_rkdg_s {
     DBuf<double> post;             // output values for the writers (allocated on first use)
     DBuf<unsigned char> post_flags;
     DBuf<int2> halo;
-    DBuf<int4> tiles;
+    DBuf<int2> tiles;
     DBuf<int> enodes, ref_of_dev;
     DBuf<double2> xy;
     DBuf<double> nz;
@@ -1043,7 +1043,7 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
         if ((e = h->halo.alloc(std::max<size_t>(nhalo, 1))) != cudaSuccess) return cleanup_fail("alloc", e);
         if (nhalo) cudaMemcpy(h->halo.p, h->tiling.halo.data(), nhalo * sizeof(int2), cudaMemcpyHostToDevice);
         if ((e = h->tiles.alloc(h->tiling.ntiles)) != cudaSuccess) return cleanup_fail("alloc", e);
-        cudaMemcpy(h->tiles.p, h->tiling.tiles.data(), h->tiling.ntiles * sizeof(int4), cudaMemcpyHostToDevice);
+        cudaMemcpy(h->tiles.p, h->tiling.tiles.data(), h->tiling.ntiles * sizeof(int2), cudaMemcpyHostToDevice);
         std::vector<double2> xy(h->nn);
         std::vector<double> nz(h->nn);
         for (int64_t i = 0; i < h->nn; ++i) {
@@ -1102,7 +1102,7 @@ static int32_t create_impl(const dgsw_config* cfg, const dgsw_mesh* mesh, const 
             if ((e = h->l2rule.alloc(1)) != cudaSuccess) return cleanup_fail("alloc", e);
             cudaMemcpy(h->l2rule.p, &Rh, sizeof(L2Rule), cudaMemcpyHostToDevice);
         }
-        h->device_bytes += en.size() * 4 + nb.size() * 4 + h->nn * 24 + h->tiling.ntiles * 16 + nhalo * 8 + h->ne * 4 + 3 * h->ne_pad;
+        h->device_bytes += en.size() * 4 + nb.size() * 4 + h->nn * 24 + h->tiling.ntiles * 8 + nhalo * 8 + h->ne * 4 + 3 * h->ne_pad;
     }
     if (cfg->slope_limiting) {
         // the limiter's geometry, once (the same device code the limiter would run per stage)

@@ -526,7 +526,7 @@ int build_tiling(const Topology& T, const double* X, int tile, bool morton, Tili
     out.dev_of_ref.resize(ne);
     for (int64_t d = 0; d < ne; ++d) out.dev_of_ref[out.ref_of_dev[d]] = (int32_t)d;
     out.ntiles = (ne + tile - 1) / tile;
-    out.tiles.assign((size_t)4 * out.ntiles, 0);
+    out.tiles.assign((size_t)2 * out.ntiles, 0);
     out.fmeta.resize((size_t)3 * ne);
     out.fw.resize((size_t)3 * ne);
     out.halo.clear();
@@ -589,7 +589,7 @@ int build_tiling(const Topology& T, const double* X, int tile, bool morton, Tili
                 out.fw[at] = sJ / J[4];
             }
         }
-        out.tiles[4 * t + 1] = (int32_t)(halo.size() / 2);
+        out.tiles[2 * t + 1] = (int32_t)(halo.size() / 2);
         // boundary faces after the halo faces: tide / flow faces carry their forcing record
         for (size_t k = 0; k < boundary.size(); k += 2) {
             const int32_t d = boundary[k], f = boundary[k + 1];
@@ -603,13 +603,12 @@ int build_tiling(const Topology& T, const double* X, int tile, bool morton, Tili
             halo.push_back(kind == EK_TIDE || kind == EK_FLOW ? T.bnd_force[bi] : -1);
             halo.push_back(0);
         }
-        out.tiles[4 * t + 2] = (int32_t)(halo.size() / 2);
     }
     out.n_edges = n_edges;
     // offsets by a prefix sum over the tiles, then every tile copies its list into place
     int64_t total = 0;
     for (int64_t t = 0; t < out.ntiles; ++t) {
-        out.tiles[4 * t] = (int32_t)total;
+        out.tiles[2 * t] = (int32_t)total;
         total += (int64_t)lists[t].size() / 2;
         out.max_halo = std::max(out.max_halo, (int)(lists[t].size() / 2));
         if (total >= std::numeric_limits<int32_t>::max()) {
@@ -620,7 +619,7 @@ int build_tiling(const Topology& T, const double* X, int tile, bool morton, Tili
     out.halo.resize((size_t)2 * total);
 #pragma omp parallel for schedule(dynamic, 64)
     for (int64_t t = 0; t < out.ntiles; ++t) {
-        std::copy(lists[t].begin(), lists[t].end(), out.halo.begin() + 2 * (int64_t)out.tiles[4 * t]);
+        std::copy(lists[t].begin(), lists[t].end(), out.halo.begin() + 2 * (int64_t)out.tiles[2 * t]);
         std::vector<int32_t>().swap(lists[t]);
     }
     return DGSW_OK;

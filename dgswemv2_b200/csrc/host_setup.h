@@ -103,8 +103,7 @@ struct Tiling {
     // Trace slots: 3*(element - tile start) + face for tile elements, 3*tile + h for entry h of the tile's list.
     bigvec<int32_t> fmeta;
     bigvec<double> fw;                   // [3 * ne] half the face's length over the element's |J|
-    // per tile: offset into halo, halo faces, halo + boundary faces, 0
-    std::vector<int32_t> tiles;          // [4 * ntiles]
+    std::vector<int32_t> tiles;          // [2 * ntiles]: per tile its offset into halo and its halo faces
     // [2 * n]: per tile its halo faces (device element, face), then its boundary faces (forcing record or -1, 0)
     bigvec<int32_t> halo;
     int64_t n_edges = 0;                 // edges of all tiles (one between two tiles counts for both)

@@ -121,10 +121,9 @@ struct DevStatus {
 
 constexpr int SINE_NCONST = 10;
 
-// What a stage needs of its time (t + dt drk[s]): the function set's time factors and the forcing ramp
+// What a stage needs of its time (t + dt drk[s]): the function set's time factors
 struct StageTime {
     dgsw_fn_time ft;
-    double ramp;
     double sine[SINE_NCONST];  // the manufactured sine set's constants (SineSrc), in both precisions
     float sine_f[SINE_NCONST];
 };
@@ -195,7 +194,6 @@ static __device__ __noinline__ void form_step_time(const TimeArgs* Tp, int block
         const int s = threadIdx.x;
         if (s < T.nstages) {
             T.next->at[s].ft = dgsw_fn_prepare(T.fn_set, T.fn_params, t + T.off[s]);
-            T.next->at[s].ramp = forcing_ramp(T, t + T.off[s]);
             if (T.fn_set == DGSW_FN_MANUFACTURED_SINE) sine_constants(T.fn_params, T.next->at[s]);
         }
         if (s == 0) {
@@ -243,7 +241,7 @@ struct StageArgs {
     // slot across the face (a neighbour's, or the boundary face's ghost slot), or the levee interface's index
     const int* fmeta;           // [3][ne_pad]
     const Real* fw;             // [3][ne_pad] half the face's length over the element's |J|
-    const int4* tiles;          // per tile: offset into halo, halo faces, halo + boundary faces
+    const int2* tiles;          // per tile: offset into halo, halo faces
     const int2* halo;           // tile lists: (element, face) per halo face, then (forcing record, 0) per boundary face
     const double2* xy;          // node coordinates
     const double* nz;           // node bathymetry depth (wet/dry vertex depths)
@@ -1217,7 +1215,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
     // manufactured 4.15 -> 3.54, bowl 2.91 -> 2.43. (Staged in the halo face's own trace slot, which takes no memory, p = 1
     // 0.92 ms; tiles sized to the mesh run 10 to 15 % slower with copies than with loads.)
     constexpr bool ASYNC = CAPPED && SM::staged;
-    const int4 ti = A.tiles[tile];
+    const int2 ti = A.tiles[tile];
     const int hoff = ti.x, nh = ti.y;
     // FP64: one thread asks L2 for the rows this CTA reads only at its end, the RK combination's earlier
     // stages, so that those loads start on L2 hits instead of HBM latency. Bulk prefetches want 16-byte aligned
