@@ -681,3 +681,50 @@ def test_tile_edges_and_remainders(oracle, nx, ny, p, tile):
     P.step_serial(9)
     O.step(13)
     assert rel_err(P.get_state(), O.get_state()) <= 1e-12
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (9, 7), (8, 8), (13, 5), (64, 2)])
+@pytest.mark.parametrize("p,tile", [(1, 128), (1, 256), (2, 128), (2, 256)])
+def test_tile_edges_and_remainders_fp32(oracle, nx, ny, p, tile):
+    """The same meshes in FP32, at p = 2 with stage increments (its own kernel) and with FP64 stage states: ghost slots
+    behind the halo slots, halo copies by threads past the last element, the p = 2 faces' run-time table. A step changes a
+    mode by dt / dx (at most 0.5 / 150) times flux and volume terms of up to g ze h = 2, some ten of them, each within a
+    few 2^-24: 13 steps leave up to 13 x 10 x 0.0033 x 2 x 2^-23 = 1e-7, 5e-6 of the smallest scale (ze, 0.02) if all
+    add up, a tenth of it as they come. Bar: 2e-6 (measured 2e-7). A wrong slot moves a flux by a part of itself, 1e-3 of
+    the scale in one stage."""
+    rk, jitter = ((2, 2) if p == 1 else (3, 3)), (0.1 if nx > 1 else 0.0)
+    mesh, cfg64 = configs.tidal_channel(nx, ny, p=p, rk=rk, dt=0.5, jitter=jitter)
+    cfg = configs.tidal_channel(nx, ny, p=p, rk=rk, dt=0.5, jitter=jitter, precision="fp32")[1]
+    O = oracle.problem(cfg64, mesh)
+    q = np.random.default_rng(5).uniform(-0.02, 0.02, (mesh.n_elems, 3, (p + 1) * (p + 2) // 2))
+    q[:, 1:] *= 10.0
+    O.set_state(q)
+    O.step(13)
+    for fp64_stages in (False, True) if p == 2 else (True,):
+        P = Problem(cfg, mesh, tile=tile, fp64_stages=fp64_stages)
+        assert bool(P.info.stage_increments) != fp64_stages
+        P.set_state(q)
+        P.step_serial(3)
+        for _ in range(cfg.rk_nstages):
+            P.stage_serial()
+        P.step_serial(9)
+        e = rel_err(P.get_state(), O.get_state())
+        assert e <= 2e-6, (fp64_stages, e)
+
+
+@pytest.mark.parametrize("p,rk", [(1, (2, 2)), (2, (3, 3))])
+def test_fp32_closed_basin_mass(p, rk):
+    """Both elements of an interface evaluate its flux, each with its own scaled normal, so that their mass fluxes cancel
+    to the rounding of the element geometry (2e-7 of the flux in FP32). 4,000 steps of a sloshing hump in a closed basin
+    over uneven bottom, jittered mesh: the mass drifts by 6e-11 of itself (1e-9 with one rounded flux per edge and two
+    rounded weights). Bar: 1e-9."""
+    bath = meshgen.bath_gaussians(3, ((0, 1e4), (0, 1e4)))
+    mesh = meshgen.quad_mesh(48, 48, corners=((0, 0), (1e4, 0), (1e4, 1e4), (0, 1e4)), bc=(LAND,) * 4, jitter=0.2, seed=5,
+                             bathymetry=bath)
+    cfg = configs.ensemble_member(8, 1, precision="fp32")[1]
+    cfg.p, cfg.rk_nstages, cfg.rk_order, cfg.wetting_drying = p, rk[0], rk[1], False
+    P = Problem(cfg, mesh)
+    m0, q0 = P.mass(), P.get_state()
+    P.step_serial(4000)
+    assert np.abs(P.get_state()[:, 1:]).max() > 0.1 and np.abs(P.get_state() - q0).max() > 0.1  # it sloshes
+    assert abs(P.mass() / m0 - 1) <= 1e-9, P.mass() / m0 - 1
