@@ -28,13 +28,14 @@ sys.path.insert(0, ROOT)
 METRIC = "element-DOF updates/s per RK stage, FP32+MLP vs FP64 plain on B200 at equal L2"
 UNIT = "element-DOF/s"
 # compulsory HBM bytes per element-DOF per RK stage (each array touched once), p = 2 SSP-RK3 and p = 1
-# SSP-RK2, keyed (precision, p, stage increments): element geometry and bathymetry (FP32 in the FP32 path)
-# and the edge records, plus the stage states. FP64 stage states: q_s read, q_{s+1} written, q_0 read by
+# SSP-RK2, keyed (precision, p, stage increments): the mesh data of an element plus the stage states. Mesh data: J^-1 (4
+# values), bathymetry (3), face weights (3) in the path's precision, face records (12 B), wet flags (2 B) and the tile's
+# halo list (about 2.4 B), 56 B in FP32 and 96 B in FP64. FP64 stage states: q_s read, q_{s+1} written, q_0 read by
 # the stages after the first. FP32 stage increments: the carried state's leading FP32 part q0f (4 B) and the
 # increment d_s (4 B) read, d_{s+1} (4 B) written; the last stage also reads the trailing part q0lo (4 B)
 # and writes both parts of the new carried state (8 B).
-ALG_BYTES_PER_UNIT = {("fp32", 2, 0): 77.0, ("fp64", 2, 0): 87.0, ("fp32", 1, 0): 82.0, ("fp64", 1, 0): 99.0,
-                      ("fp32", 2, 1): 53.0}
+ALG_BYTES_PER_UNIT = {("fp32", 2, 0): 73.0, ("fp64", 2, 0): 80.0, ("fp32", 1, 0): 79.0, ("fp64", 1, 0): 92.0,
+                      ("fp32", 2, 1): 49.0}
 
 
 def workload_name(nq, ne):

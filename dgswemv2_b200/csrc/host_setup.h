@@ -1,5 +1,5 @@
 // Host-side preprocessing of the RKDG library: mesh topology in the reference's order, the element
-// permutation and CTA tiling used on the device, per-tile edge lists, master tables and the FP64
+// permutation and CTA tiling used on the device, face records and per-tile halo lists, master tables and the FP64
 // initial projections. Host C++ only.
 #ifndef DGSW_HOST_SETUP_H
 #define DGSW_HOST_SETUP_H

@@ -6,25 +6,28 @@
 //      memory. Neighbours in other tiles ("halo" faces) get their face traces written by the same routine
 //      from global memory, and a boundary face's ghost state (BC::Land / Tide / Flow / Function,
 //      rkdg_swe_bc_land.hpp:41-66, rkdg_swe_bc_function.hpp:27-60) goes to a trace slot of its own, so that the
-//      face loop below has no boundary branches. Then the thread arrives on the CTA's one barrier;
+//      face loop below has no boundary branches. Then the thread arrives on the barrier between the traces and the
+//      faces (the only other one follows the CTA's set-up, before any trace);
 //   2. accumulates the volume and source integrals in registers (Problem::volume_kernel + source_kernel,
 //      rkdg_swe_proc_volume.hpp:9-35, rkdg_swe_proc_source.hpp:9-18) while the other warps' traces arrive;
 //   3. waits on the barrier and takes the numerical flux of its own three faces (LLF + the wet/dry fix-ups of
 //      ISP::Internal, rkdg_swe_is_internal.hpp:26-95) straight into the lift. Both elements of an interface
-//      evaluate the flux, each with its outward normal; the formula is arranged so that the two are exact
-//      negatives of each other, as in the reference;
+//      evaluate the flux, each with the outward normal and the weight of its own geometry. For one shared normal the
+//      formula's two values are exact negatives, as the reference's are; here they cancel to the rounding of J^-1,
+//      2e-7 of the flux in FP32, and a mass flux that is itself rounding may be refused by a dry side and given by
+//      the wet one. Mass of a closed basin after 4,000 steps: 6e-11 off in FP32, 4e-15 in FP64;
 //   4. applies M^-1 and the SSP-RK stage combination (element.hpp:502-505,
 //      explicit_ssp_rk_stepper.hpp:67-80), the wetting/drying kernel (swe_post_wet_dry.hpp:6-145, its depth
 //      tests in FP64 in every precision) and the NaN scrutiny; writes the next stage state.
-// What bounds it: latency and instruction issue, not bytes (20-35 % of the HBM rate), so it is arranged for few
+// What bounds it: latency and instruction issue, not bytes (15 to 46 % of the HBM rate), so it is arranged for few
 // instructions and few waits. Evaluating each flux twice costs about four more LLF evaluations per element than
 // one per edge of the tile, and saves the flux's way through shared memory, the edge lists, a second barrier and the
-// half-empty second round of edges. Against one flux per edge between two barriers, 524,288 triangles, p = 2, FP32:
-// warp instructions of the second stage 46.7 M -> 33.9 M, barrier stalls 1.3 -> 0.1 per issue, cold 97.7 -> 77.9 us;
-// 8 steps 2.36 -> 1.95 ms (FP64 4.74 -> 4.18 ms); tidal channel p = 1 of 433,394 FP32 0.74 -> 0.56 ms; ensemble of 24
-// wet/dry members FP32 1.84 -> 1.42 ms.
-// The master tables are compile-time constants (tables_gen.h): every table entry is an immediate,
-// zero entries are skipped and unit entries become additions.
+// half-empty second round of edges. Against one flux per edge between two barriers, and with the step time formed once
+// per step: 524,288 triangles, p = 2, FP32, second stage: warp instructions 46.7 M -> 35.4 M, barrier stalls 1.3 -> 0.1
+// per issue, cold 97.7 -> 73.6 us; 8 steps 2.43 -> 1.89 ms (FP64 4.81 -> 3.70 ms); tidal channel p = 1 of 433,394 FP32
+// 0.84 -> 0.54 ms; ensemble of 24 wet/dry members FP32 1.95 -> 1.30 ms.
+// The master tables are compile-time constants (tables_gen.h): in the unrolled loops every table entry is an immediate and
+// zero entries are skipped; the rolled ones read them from constant memory (stage_tab).
 // HBM layout: component-major SoA, q[(var*ND + dof) * ne_pad + element].
 #ifndef DGSW_STAGE_KERNEL_CUH
 #define DGSW_STAGE_KERNEL_CUH
@@ -340,7 +343,7 @@ __device__ __forceinline__ void complete(Side<Real>& s, Real g) {
 // The LLF flux above (sp = 1) of the own side towards the neighbour n, doubled and times w, along the own
 // outward normal times w, N = w nrm: with qn = q . N and un = qn / h the normal flux of a side is
 // (qn, q un + pe N), the same terms as above with the products regrouped (a few ulps). Every term changes sign
-// exactly when the sides trade places and the normal turns round.
+// exactly when the sides trade places and the same N turns round.
 template <bool PK, typename Real>
 __device__ __forceinline__ void llf_sides(Real g, const Side<Real>& o, const Side<Real>& n, Two<Real> N, Real w, Real& F0,
                                           Two<Real>& F12) {
@@ -397,7 +400,7 @@ struct Val3 {
     Real v0, v1, v2;
 };
 
-// analytic function sets evaluated out of line (one copy per kernel); T points to the CTA's shared copy
+// analytic function sets evaluated out of line (one copy per kernel); T: the stage's time factors
 template <typename Real>
 __device__ __noinline__ Val3<Real> fn_eval_dev(int id, const double* P, const dgsw_fn_time* T, int source, Real x,
                                                Real y) {
@@ -801,7 +804,7 @@ __device__ __noinline__ void ghost_face(const StageArgs<Real>* Ap, unsigned char
 // The spherical correction cos(phi_0) / cos(y / R) at an element's face and volume Gauss points (geometry alone):
 // rows face * NG + gp, then 3 NG + gp, of [ne_pad] values, formed once per handle. In the stage kernel it was a cosine in
 // FP64 per point, and two per face point as both elements of a face evaluate its flux. 8 steps of 131,072 triangles:
-// tidal channel p = 1 FP64 0.71 -> 0.44 ms, FP32 0.43 -> 0.28, p = 2 FP64 2.09 -> 1.41, FP32 0.99 -> 0.63; wet/dry bowl
+// tidal channel p = 1 FP64 0.71 -> 0.38 ms, FP32 0.43 -> 0.28, p = 2 FP64 2.09 -> 1.29, FP32 0.99 -> 0.64; wet/dry bowl
 // p = 1 FP64 0.76 -> 0.38, FP32 0.39 -> 0.24.
 template <int P>
 constexpr int spherical_rows() {
@@ -994,12 +997,14 @@ __device__ __forceinline__ void cp_async_commit_and_wait() {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// resident CTAs per SM the register budget is sized for (p = 1 and p = 2 separately; measured at tile
-// 128 on 524,288 triangles: p = 2 FP32 4 (5 spills 592 B and runs 40 % slower), p = 1 FP32 5 (3-9 %
-// faster than 4 on the bowl, tidal, levee and manufactured workloads; 6 spills and is slower), p = 2
-// FP64 3, p = 1 FP64 4 without wetting/drying or analytic source (the tidal channel 0.96 against 1.07 ms per 8
-// steps), 3 with the source (4 spills: 1.63 against 1.36 ms) and with wetting/drying (bowl of 131,072 0.55 against
-// 0.57 ms; of 980,000 3.10 against 2.86 ms, but 3 for the smaller ones))
+// resident CTAs per SM the register budget is sized for (p = 1 and p = 2 separately; tile 128, per 8 steps): p = 2 FP32 4
+// (5 spills 592 B and runs 40 % slower), p = 1 FP32 5 (3-9 % faster than 4 on the bowl, tidal, levee and manufactured
+// workloads; 6 spills and is slower), p = 2 FP64 3. p = 1 FP64: 4 without wetting/drying or analytic source (tidal channel
+// of 524,288 0.97 against 1.11 ms with 3; below about 50,000, one wave either way, 3 is up to 8 % faster); 3 with the
+// source (manufactured of 524,288 1.29 against 1.31 ms with 4, of 32,768 0.19 against 0.23; 4 wins where it saves the last
+// wave, of 65,522 0.28 against 0.30); 3 with wetting/drying, which suits small meshes only (bowl of 8,192 0.193 against
+// 0.206 ms, of 32,768 0.200 against 0.210, but of 131,072 0.34 against 0.33, of 524,288 1.01 against 0.91 and of 1,048,352
+// 1.99 against 1.76): a budget by the number of waves is not built
 #ifndef DGSW_F32_MB128
 #define DGSW_F32_MB128 4
 #endif
@@ -1029,15 +1034,16 @@ struct MinBlocks {
     static constexpr int value = OCC == 0 ? base : (base > 1 ? base - 1 : base + 1);
 };
 
-// shared-memory capacity a tile almost always fits (measured: about 0.27 TILE halo faces on structured and
-// jittered meshes); with CAPPED the stride of the trace vectors is this compile-time constant, so every
-// shared-memory access has an immediate offset
+// shared-memory capacity; with CAPPED the stride of the trace vectors is this compile-time constant, so every
+// shared-memory access has an immediate offset. On quad meshes whose sides are powers of two a tile of 128 has 35 halo
+// and boundary faces on average and 56 at most; with other sides (the Morton order cuts them into less compact tiles)
+// 57 and 86, and those run with strides read at run time
 template <int TILE>
 struct TileCap {
     static constexpr int halo = TILE / 2;
 };
 
-// the CTA's one barrier: warps arrive with their traces written and wait after the volume integral
+// the barrier between traces and faces: warps arrive with their traces written and wait after the volume integral
 __device__ __forceinline__ void stage_bar_init(unsigned long long* bar, unsigned warps) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(warps)
                  : "memory");
@@ -1146,7 +1152,8 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
     // FP64 p = 2). Measured per 8 steps of 524,288 triangles, unrolled -> rolled: FP64 p = 2 5.08 -> 4.53 ms (points)
     // -> 4.34 ms (points and faces), FP64 p = 1 manufactured 1.41 -> 1.36 ms, the FP64 bowl of 980,000 3.34 -> 3.25 ms;
     // FP32 p = 2 faces 2.08 -> 2.05 ms, points 2.08 -> 2.22 ms; FP32 p = 1 manufactured, points and faces,
-    // 0.735 -> 0.749 ms; FP64 p = 1 channel 0.96 -> 1.00 ms or more. So the FP32 points and all of FP32 p = 1 stay
+    // 0.735 -> 0.749 ms; FP64 p = 1 channel 0.96 -> 1.00 ms or more; FP64 p = 2 without a source, closed basin 3.38 ->
+    // 3.29 and channel 3.90 -> 3.60 ms (all with FP64's halo elements staged in shared memory, see below). So the FP32 points and all of FP32 p = 1 stay
     // unrolled, and FP64 p = 1 without source and wetting/drying.
     constexpr bool ROLL_V = sizeof(Real) == 8 && (P == 2 || FSRC || WD);
     constexpr bool ROLL_F = P == 2 || (sizeof(Real) == 8 && (FSRC || WD));
@@ -1292,8 +1299,8 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
     Real q[3][ND], b[3];
     Real Ji00 = Real(0), Ji01 = Real(0), Ji10 = Real(0), Ji11 = Real(0);
     Real x0 = 0, y0 = 0, x1 = 0, y1 = 0, x2 = 0, y2 = 0;
-    // the vertex coordinates (analytic source). FP64 at p = 2, whose register budget is
-    // tightest, loads them after the traces
+    // the vertex coordinates (analytic source). FP64 at p = 2, whose register budget is tightest, loads them after the
+    // traces
     constexpr bool xy_early = sizeof(Real) == 4 || P == 1;
     auto load_xy = [&]() {
         if (FSRC) {
@@ -1772,8 +1779,8 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
         if (A.last) {
             // the new carried state q0f + q0lo + d_ns in FP64 (q0f + q0lo is exact there), split again into
             // its leading and trailing Real parts; q_0 is loaded here rather than with the increments (held
-            // across the edge gather its registers would spill; its leading part is an L1 or L2 hit from
-            // phase 1)
+            // across the face loop its registers would spill; its leading part is an L1 or L2 hit from the
+            // traces)
             Real hi[3][ND], lo[3][ND];
 #pragma unroll
             for (int v = 0; v < 3; ++v)
