@@ -1000,7 +1000,7 @@ __device__ __forceinline__ void cp_async_commit_and_wait() {
 // resident CTAs per SM the register budget is sized for (p = 1 and p = 2 separately; tile 128, per 8 steps): p = 2 FP32 4
 // (5 spills 592 B and runs 40 % slower), p = 1 FP32 5 (3-9 % faster than 4 on the bowl, tidal, levee and manufactured
 // workloads; 6 spills and is slower), p = 2 FP64 3. p = 1 FP64: 4 without wetting/drying or analytic source (tidal channel
-// of 524,288 0.97 against 1.11 ms with 3; below about 50,000, one wave either way, 3 is up to 8 % faster); 3 with the
+// of 524,288 0.94 against 1.11 ms with 3; one wave either way, 32,768, 0.154 against 0.155); 3 with the
 // source (manufactured of 524,288 1.29 against 1.31 ms with 4, of 32,768 0.19 against 0.23; 4 wins where it saves the last
 // wave, of 65,522 0.28 against 0.30); 3 with wetting/drying, which suits small meshes only (bowl of 8,192 0.193 against
 // 0.206 ms, of 32,768 0.200 against 0.210, but of 131,072 0.34 against 0.33, of 524,288 1.01 against 0.91 and of 1,048,352
@@ -1218,7 +1218,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
     // FP64 loads the halo elements after its own traces, in every tile: the staging area, 6 KB (p = 1) or 11 KB (p = 2) a
     // CTA, put the resident CTAs' shared memory above 196 KB, which leaves the L1 28 KB for 512 or 384 threads' loads in
     // flight instead of 60. Measured per 8 steps of 524,288 triangles, with staging -> without: p = 1 closed basin 1.17 ->
-    // 0.84 ms, channel 1.25 -> 0.96, bowl 1.03 -> 1.02; p = 2 closed basin 3.29 -> 2.68 ms, channel 3.60 -> 2.95,
+    // 0.84 ms, channel 1.25 -> 0.97, bowl 1.03 -> 1.02; p = 2 closed basin 3.29 -> 2.68 ms, channel 3.60 -> 2.95,
     // manufactured 4.15 -> 3.54, bowl 2.91 -> 2.43. (Staged in the halo face's own trace slot, which takes no memory, p = 1
     // 0.92 ms; tiles sized to the mesh run 10 to 15 % slower with copies than with loads.)
     constexpr bool ASYNC = CAPPED && SM::staged;
@@ -1334,9 +1334,10 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
             swet[3 * tid + f] = wet ? 1 : 0;
         });
         // boundary faces: their ghost states. A dry element's has no flux. One call site for the three faces, as few
-        // elements have such a face and almost none two; FP32 at p = 1 keeps three (the loop makes it spill: manufactured
-        // of 1,048,352, 8 steps, 1.36 against 1.22 ms). Boundary-heavy FP64 meshes, 8 steps: 8,000 wet/dry members of 18
-        // triangles 0.50 -> 0.42 ms, 1,000 of 200 0.60 -> 0.52, with this, the one division and the kept 1 / h.
+        // elements have such a face and almost none two; at p = 1 FP32 and plain FP64, whose registers are tightest, keep
+        // three (with the loop FP32 spills: manufactured of 1,048,352, 8 steps, 1.36 against 1.22 ms; FP64 closed basin of
+        // 1,048,352 1.79 against 1.67, of 2,048 0.130 against 0.118). Boundary-heavy FP64 meshes, 8 steps: 8,000 wet/dry
+        // members of 18 triangles 0.50 -> 0.42 ms, 1,000 of 200 0.60 -> 0.52, with this, the one division and the kept 1 / h.
         auto ghost = [&](auto FF, int m, Real w) {
             const auto fc = FF;
             const int f = fc;
@@ -1346,7 +1347,7 @@ __global__ void __launch_bounds__(TILE, (MinBlocks<P, Real, TILE, WD, FSRC, OCC>
             const Two<Real> N = scaled_normal<Real>(f, Ji00, Ji01, Ji10, Ji11);
             ghost_face<P, Real>(&A, tr, NS, 3 * tid + f, slot, d, f, kind, A.halo[hoff + slot - 3 * TILE].x, N.x, N.y, w);
         };
-        if constexpr (sizeof(Real) == 8 || P == 2) {
+        if constexpr (P == 2 || (sizeof(Real) == 8 && (WD || FSRC))) {
             int bnd = 0;
 #pragma unroll
             for (int f = 0; f < 3; ++f) {
